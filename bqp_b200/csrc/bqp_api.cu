@@ -93,14 +93,15 @@ bool parse_coeffs(const char* text, int64_t len, int order, Coeffs& out, std::st
     return true;
 }
 
-// Per-cell table of the normalised column recursion (see gravity.cuh).  The
-// C00 term is left out: the propagator removes the central term analytically
+// Cells of the normalised column recursion (see gravity.cuh), columns
+// ascending, kCellDoubles numbers each: a, b and the six weights.  The C00
+// term is left out: the propagator removes the central term analytically
 // (rhs.rs:2735-2744, 2849-2855), which is what dropping it computes exactly.
-std::vector<double> build_gravity_table(const Coeffs& cf, int order) {
+std::vector<long double> gravity_cell_values(const Coeffs& cf, int order) {
     typedef long double LD;
     const int N = order;
     const int ncells = gravity_cells(N);
-    std::vector<double> tab((size_t)ncells * kCellDoubles, 0.0);
+    std::vector<LD> tab((size_t)ncells * kCellDoubles, 0.0L);
     const int ld = cf.order + 1;
     auto C = [&](int n, int k) -> LD {
         if (n < 0 || k < 0 || k > n || n > N) return 0.0L;
@@ -127,7 +128,7 @@ std::vector<double> build_gravity_table(const Coeffs& cf, int order) {
     size_t cell = 0;
     for (int j = 0; j <= N + 1; ++j) {
         for (int l = j; l <= N + 1; ++l, ++cell) {
-            double* o = &tab[cell * kCellDoubles];
+            LD* o = &tab[cell * kCellDoubles];
             LD a = 0.0L, b = 0.0L;
             if (l == j) {
                 a = (j == 0) ? 0.0L : (j == 1 ? std::sqrt(3.0L) : std::sqrt((2.0L * j + 1) / (2.0L * j)));
@@ -170,16 +171,57 @@ std::vector<double> build_gravity_table(const Coeffs& cf, int order) {
                     Bz += -w * S(n, j) * r;
                 }
             }
-            o[0] = (double)a;
-            o[1] = (double)b;
-            o[2] = (double)(Ax * gm_r2);
-            o[3] = (double)(Bx * gm_r2);
-            o[4] = (double)(Ay * gm_r2);
-            o[5] = (double)(By * gm_r2);
-            o[6] = (double)(Az * gm_r2);
-            o[7] = (double)(Bz * gm_r2);
+            o[0] = a;
+            o[1] = b;
+            o[2] = Ax * gm_r2;
+            o[3] = Bx * gm_r2;
+            o[4] = Ay * gm_r2;
+            o[5] = By * gm_r2;
+            o[6] = Az * gm_r2;
+            o[7] = Bz * gm_r2;
         }
     }
+    return tab;
+}
+
+// The FP64 table of gravity_part: every column's recursion divided by the
+// constants s(l, j) that make its first cell and its second coefficient one
+// (s(j,j) the sectoral factor, s(j+1,j) = a s(j,j), s(l,j) = b s(l-2,j)), the
+// weights times them.
+std::vector<double> build_gravity_table(const std::vector<long double>& cells, int order) {
+    typedef long double LD;
+    std::vector<double> tab;
+    tab.reserve(gravity_tab_doubles(order) + kGravityTabPad);
+    const int last = order + 1;
+    LD sect = 1.0L;
+    for (int j = 0; j <= last; ++j) {
+        const LD* col = &cells[(size_t)gravity_col_offset(order, j) * kCellDoubles];
+        if (j > 0) sect *= col[0];
+        std::vector<LD> s(order + 2 - j);
+        for (int k = 0; k < (int)s.size(); ++k) {
+            const LD* o = col + (size_t)k * kCellDoubles;
+            s[k] = k == 0 ? sect : (k == 1 ? o[0] * s[0] : o[1] * s[k - 2]);
+        }
+        auto weights = [&](int k) {
+            for (int i = 2; i < kCellDoubles; ++i)
+                tab.push_back((double)(col[(size_t)k * kCellDoubles + i] * s[k]));
+        };
+        auto coef = [&](int k) { tab.push_back((double)(col[(size_t)k * kCellDoubles] * s[k - 1] / s[k])); };
+        int k = 0;
+        for (; k < 2 && k < (int)s.size(); ++k) weights(k);
+        if ((s.size() & 1) && s.size() > 2) {
+            coef(k);
+            tab.push_back(0.0);
+            weights(k++);
+        }
+        for (; k < (int)s.size(); k += 2) {
+            coef(k);
+            coef(k + 1);
+            weights(k);
+            weights(k + 1);
+        }
+    }
+    tab.resize(tab.size() + kGravityTabPad, 0.0);
     return tab;
 }
 
@@ -788,7 +830,8 @@ CtrlParams ctrl_params(const bqp_ctx* ctx) {
 }
 
 int upload_table(bqp_ctx* ctx) {
-    std::vector<double> tab = build_gravity_table(ctx->coeffs, ctx->cfg.order);
+    const std::vector<long double> cells = gravity_cell_values(ctx->coeffs, ctx->cfg.order);
+    const std::vector<double> tab = build_gravity_table(cells, ctx->cfg.order);
     ctx->ncells = gravity_cells(ctx->cfg.order);
     ctx->tab_bytes = tab.size() * sizeof(double);
     ctx->use_smem = ctx->tab_bytes <= kSmemLimit ? 1 : 0;
@@ -812,14 +855,14 @@ int upload_table(bqp_ctx* ctx) {
         for (int j = 0; j <= last; ++j) {
             const size_t col = (size_t)gravity_col_offset(N, j);
             for (int l = j; l <= last; ++l) {
-                const double* c = &tab[(col + (l - j)) * kCellDoubles];
+                const long double* c = &cells[(col + (l - j)) * kCellDoubles];
                 if (j <= ls && l <= ls) {
                     double* o = lo + ((size_t)split_lo_offset(ls, j) + (l - j)) * kCellDoubles;
-                    for (int k = 0; k < kCellDoubles; ++k) o[k] = c[k];
+                    for (int k = 0; k < kCellDoubles; ++k) o[k] = (double)c[k];
                 } else {
                     const int first = j <= ls ? ls + 1 : j;  // first FP32 row of column j
                     float* o = hi + ((size_t)split_hi_offset(N, ls, j) + (l - first)) * kCellDoubles;
-                    for (int k = 0; k < kCellDoubles; ++k) o[k] = (float)c[k];
+                    for (int k = 0; k < kCellDoubles; ++k) o[k] = (float)(double)c[k];
                 }
             }
         }
@@ -843,12 +886,10 @@ GravTable grav_table(const bqp_ctx* ctx) {
         T.tab = static_cast<const double*>(ctx->d_tab_split);
         T.ls = ctx->split_ls;
         T.bytes = ctx->split_bytes;
+        T.in_smem = T.bytes <= kSmemLimit ? 1 : 0;
     } else {
-        T.tab = ctx->d_tab;
-        T.ls = 0;
-        T.bytes = (uint32_t)ctx->tab_bytes;
+        T = gravity_table(ctx->d_tab, ctx->cfg.order);
     }
-    T.in_smem = T.bytes <= kSmemLimit ? 1 : 0;
     return T;
 }
 
@@ -909,7 +950,7 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
     A.evals = evals;
     A.queue = ctx->d_queue;
     A.gtab = ctx->d_tab;
-    A.ncells = ctx->ncells;
+    A.tab_bytes = (uint32_t)ctx->tab_bytes;
     A.use_smem = ctx->use_smem;
     if (int rc = ensure_fit2(ctx)) return rc;
     if (int rc = frame_prepare_dev(ctx, n, epoch, t0, tf)) return rc;
@@ -1580,7 +1621,7 @@ int bqp_rhs_eval_device(bqp_ctx* ctx, int64_t n, const double* equ, const double
     int rc = set_device(ctx);
     if (rc) return rc;
     if ((rc = frame_prepare_dev(ctx, n, epoch_jd, 0.0, t, t))) return rc;
-    cudaError_t e = launch_rhs(ctx->d_tab, ctx->ncells, ctx->use_smem, force_params(ctx), n, equ, seg_t0,
+    cudaError_t e = launch_rhs(ctx->d_tab, (uint32_t)ctx->tab_bytes, ctx->use_smem, force_params(ctx), n, equ, seg_t0,
                                epoch_jd, t, delta, ballistic, ctx->cfg.am_ratio, ctx->cfg.cd, out, ctx->stream);
     return e == cudaSuccess ? 0 : cuda_fail(e, "k_rhs launch");
 }
@@ -1616,7 +1657,7 @@ int bqp_rhs_eval(bqp_ctx* ctx, int64_t n, const double* equ, const double* seg_t
     if (e == cudaSuccess) e = cudaMemcpyAsync(dd, delta, b6, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess && db) e = cudaMemcpyAsync(db, ballistic, 2 * b1, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = launch_rhs(ctx->d_tab, ctx->ncells, ctx->use_smem, force_params(ctx), n, de, dt0, djd, dt, dd, db,
+        e = launch_rhs(ctx->d_tab, (uint32_t)ctx->tab_bytes, ctx->use_smem, force_params(ctx), n, de, dt0, djd, dt, dd, db,
                        ctx->cfg.am_ratio, ctx->cfg.cd, dout, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, dout, b6, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1895,7 +1936,7 @@ int bqp_propagate_final_noalloc(bqp_ctx* ctx, int64_t n, const double* in, int32
     A.evals = devals;
     A.queue = queue;
     A.gtab = ctx->d_tab;
-    A.ncells = ctx->ncells;
+    A.tab_bytes = (uint32_t)ctx->tab_bytes;
     A.use_smem = ctx->use_smem;
     A.force = force_params(ctx);
     // the sweep fits are built with the context and rebuilt by the calls that
@@ -2104,36 +2145,19 @@ extern "C" int bqp_gemm_bf16_device(int64_t m, int64_t n, int64_t k, const void*
 // Learned gravity surrogate (surrogate.cu).
 namespace {
 
-GravTable plain_table(const bqp_ctx* ctx) {
-    GravTable T{};
-    T.tab = ctx->d_tab;
-    T.order = ctx->cfg.order;
-    T.ls = 0;
-    T.bytes = (uint32_t)ctx->tab_bytes;
-    T.in_smem = T.bytes <= kSmemLimit ? 1 : 0;
-    return T;
-}
-
 int ensure_low_table(bqp_ctx* ctx) {
     if (ctx->d_tab_low) return 0;
     if (ctx->parsed_order < BQP_SURROGATE_DEGREE)
         return fail(BQP_E_ARG, "the surrogate needs a field of degree > %d", BQP_SURROGATE_DEGREE);
-    std::vector<double> tab = build_gravity_table(ctx->coeffs, BQP_SURROGATE_DEGREE);
+    const std::vector<double> tab =
+        build_gravity_table(gravity_cell_values(ctx->coeffs, BQP_SURROGATE_DEGREE), BQP_SURROGATE_DEGREE);
     ctx->low_bytes = (uint32_t)(tab.size() * sizeof(double));
     cudaError_t e = cudaMalloc(&ctx->d_tab_low, ctx->low_bytes);
     if (e == cudaSuccess) e = cudaMemcpy(ctx->d_tab_low, tab.data(), ctx->low_bytes, cudaMemcpyHostToDevice);
     return e == cudaSuccess ? 0 : cuda_fail(e, "surrogate low-degree table");
 }
 
-GravTable low_table(const bqp_ctx* ctx) {
-    GravTable T{};
-    T.tab = ctx->d_tab_low;
-    T.order = BQP_SURROGATE_DEGREE;
-    T.ls = 0;
-    T.bytes = ctx->low_bytes;
-    T.in_smem = 1;
-    return T;
-}
+GravTable low_table(const bqp_ctx* ctx) { return gravity_table(ctx->d_tab_low, BQP_SURROGATE_DEGREE); }
 
 int surrogate_ready(bqp_ctx* ctx, bool need_trained);
 
@@ -2183,7 +2207,7 @@ int bqp_surrogate_train(bqp_ctx* ctx, int64_t samples, int32_t epochs, int32_t b
                     ctx->cfg.order);
     if (samples < 1024 || epochs < 1 || batch < 128 || batch % 128 || batch > 65536 || !(lr > 0.0))
         return fail(BQP_E_ARG, "samples >= 1024, epochs >= 1, batch a multiple of 128 up to 65536, lr > 0");
-    const GravTable full = plain_table(ctx), low = low_table(ctx);
+    const GravTable full = gravity_table(ctx->d_tab, ctx->cfg.order), low = low_table(ctx);
     cudaStream_t s = ctx->stream;
     FieldFn ffull = [&](int64_t n, const double* pos, double* acc) {
         return launch_gravity(full, n, pos, acc, nullptr, s, 256, 4);

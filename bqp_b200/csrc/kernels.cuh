@@ -91,11 +91,11 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 
 // Copy the field table into dynamic shared memory with 16-byte vector loads.
-__device__ __forceinline__ const double* stage_table(const double* __restrict__ g, int ncells,
+__device__ __forceinline__ const double* stage_table(const double* __restrict__ g, uint32_t bytes,
                                                      bool to_smem) {
     extern __shared__ __align__(16) double smem_tab[];
     if (!to_smem) return g;
-    const int nvec = ncells * (kCellDoubles / 2);
+    const int nvec = (int)(bytes / sizeof(double2));
     const double2* src = reinterpret_cast<const double2*>(g);
     double2* dst = reinterpret_cast<double2*>(smem_tab);
     for (int i = threadIdx.x; i < nvec; i += blockDim.x) dst[i] = __ldg(src + i);

@@ -40,7 +40,7 @@ struct PropArgs {
     int64_t* evals;                // [n] or null
     unsigned long long* queue;     // work-queue head, zeroed before launch
     const double* gtab;            // gravity table (global), FP64 cells (the Encke force call)
-    int32_t ncells;
+    uint32_t tab_bytes;            // its size
     int32_t use_smem;
     GravTable grav;                // the gravity stage's table (plain or split precision)
     SurrogateRef sur;              // gravity stage through the surrogate (sur.P != null)
@@ -101,7 +101,7 @@ cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cu
 
 cudaError_t launch_gravity(const GravTable& T, int64_t n, const double* pos, double* acc, int32_t* status,
                            cudaStream_t st, int threads = 256, int slots = 4);
-cudaError_t launch_rhs(const double* gtab, int ncells, int use_smem, const ForceParams& fp, int64_t n,
+cudaError_t launch_rhs(const double* gtab, uint32_t tab_bytes, int use_smem, const ForceParams& fp, int64_t n,
                        const double* equ, const double* seg_t0, const double* jd0, const double* t,
                        const double* delta, const double* ballistic, double am0, double cd0,
                        double* out, cudaStream_t st);

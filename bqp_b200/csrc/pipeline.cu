@@ -10,8 +10,8 @@
 //   pl_prep<M>(s)   finish stage s-1, form y_s = y + h sum a_sj k_j, the Encke
 //                   baseline (Kepler solve), Earth rotation, Sun/Moon third body
 //                   and Battin's term                       (latency / SFU bound)
-//   pl_gravity      normalised column recursion, table in shared memory,
-//                   one trajectory per thread               (FP64-FMA bound)
+//   pl_gravity      normalised column recursion, table in shared memory
+//                                                           (FP64-FMA bound)
 //   pl_drag         JB2008 density and co-rotating drag     (transcendental bound)
 //   pl_control<M>   finish the last stage, error norm, accept / reject, samples,
 //                   rectification, next attempt; compacts the active list
@@ -241,18 +241,17 @@ __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cu
 }
 
 // ------------------------------------------------------------------ gravity
-// Persistent over slots: one CTA per SM stages the field table once; the
-// CTA's contiguous slot range is walked NT slots per thread.
+// Persistent over slots: every CTA (or cluster) takes an equal, contiguous
+// share of the active slots.
 // `out` receives the field; with `list` set the rows are the slots
 // list[0 .. *list_count) instead of the active slots 0 .. count.
-template <int NT>
-__global__ void __launch_bounds__(256, 1) pl_gravity(GravTable T, int parts_max, PipeBufs P, int cur, double* out,
-                                                     const int32_t* list, const int32_t* list_count) {
-    const int count = list ? *list_count : P.count[cur];
-    const int per_block = (count + gridDim.x - 1) / gridDim.x;
-    const int b0 = blockIdx.x * per_block;
-    const int b1 = min(count, b0 + per_block);
-    if (b0 >= b1) return;  // uniform across the CTA
+template <int NT, int kForm>
+__global__ void __launch_bounds__(256, 1) pl_gravity(const __grid_constant__ GravTable T, int aux, PipeBufs P, int cur,
+                                                     double* out, const int32_t* list, const int32_t* list_count) {
+    int64_t per, c0, c1;
+    gravity_rows<kForm>(list ? *list_count : P.count[cur], aux, &per, &c0, &c1);
+    const int b0 = (int)c0, b1 = (int)c1;
+    if (b0 >= b1) return;  // uniform across the CTA and its cluster
     auto load = [&](int row, double& x, double& y, double& z) -> bool {
         const int sl = list ? list[row] : row;
         if (P.skip[sl]) return false;
@@ -270,7 +269,7 @@ __global__ void __launch_bounds__(256, 1) pl_gravity(GravTable T, int parts_max,
         z = q[2];
         return true;
     };
-    auto store = [&](int row, const double* a, double, double, double) {
+    auto store = [&](int row, const double* a) {
         const int sl = list ? list[row] : row;
         out[sl] = a[0];
         out[P.cap + sl] = a[1];
@@ -281,7 +280,20 @@ __global__ void __launch_bounds__(256, 1) pl_gravity(GravTable T, int parts_max,
         P.bad[sl] = 2;
         out[sl] = out[P.cap + sl] = out[2 * P.cap + sl] = NAN;
     };
-    gravity_cta<NT>(T, parts_max, per_block, b0, b1, load, store, lost);
+    gravity_cta<NT, kForm>(T, aux, (int)per, b0, b1, load, store, lost);
+}
+
+using GravKernel = void (*)(const GravTable, int, PipeBufs, int, double*, const int32_t*, const int32_t*);
+
+template <int F>
+static GravKernel pl_gravity_form(int nt) {
+    return nt == 1 ? pl_gravity<1, F> : nt == 2 ? pl_gravity<2, F> : pl_gravity<4, F>;
+}
+
+static GravKernel pl_gravity_of(const GravLaunch& G) {
+    return G.form == kGravSplit     ? pl_gravity_form<kGravSplit>(G.nt)
+           : G.form == kGravCluster ? pl_gravity_form<kGravCluster>(G.nt)
+                                    : pl_gravity_form<kGravPlain>(G.nt);
 }
 
 // Earth-fixed positions of the stage's active slots, [slot][3] (the
@@ -606,34 +618,19 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     constexpr int kLanesHigh = BQP_DRAG_LANES_HIGH, kLanesLow = BQP_DRAG_LANES_LOW;
     const int dblocks_hi = (int)((A.n * kLanesHigh + kBlock - 1) / kBlock);
     const int dblocks_lo = (int)((A.n * kLanesLow + kBlock - 1) / kBlock);
-    const int nt = gslots == 1 || gslots == 2 ? gslots : 4;
-    auto gker = nt == 1 ? pl_gravity<1> : (nt == 2 ? pl_gravity<2> : pl_gravity<4>);
-    if (gthreads > 256) gthreads = 256;
-    if (gthreads < 32) gthreads = 32;
-    gthreads = gthreads / 32 * 32;
-    // column groups need room for their partial sums next to the table
-    int gparts = kGravityPartsMax;
     // with the surrogate, the exact stage covers only the degrees it leaves out
     const bool sur = A.sur.P != nullptr;
     const GravTable GT = sur ? A.sur.low : A.grav;
-    size_t smem = gravity_smem_bytes(GT, gthreads, nt, gparts);
-    if (smem > kSmemPerBlock) {
-        gparts = 1;
-        smem = gravity_smem_bytes(GT, gthreads, nt, gparts);
-    }
     // the surrogate's residual check also runs the whole exact field
     const bool check = sur && A.sur.check > 0.0;
-    int gparts_full = kGravityPartsMax;
-    size_t smem_full = 0;
-    if (check) {
-        smem_full = gravity_smem_bytes(A.sur.full, gthreads, nt, gparts_full);
-        if (smem_full > kSmemPerBlock) {
-            gparts_full = 1;
-            smem_full = gravity_smem_bytes(A.sur.full, gthreads, nt, gparts_full);
-        }
-    }
-    cudaError_t e = cudaFuncSetAttribute(gker, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(smem > smem_full ? smem : smem_full));
+    GravLaunch G = gravity_launch(GT, A.n, device_sm_count(), gthreads, gslots);
+    GravLaunch GF = check ? gravity_launch(A.sur.full, A.n, device_sm_count(), gthreads, gslots) : G;
+    auto gker = pl_gravity_of(G), gker_full = pl_gravity_of(GF);
+    // the larger shared memory last: the two may be one kernel
+    cudaError_t e = cudaSuccess;
+    if (check && GF.smem < G.smem) e = gravity_ready(GF, gker_full);
+    if (e == cudaSuccess) e = gravity_ready(G, gker);
+    if (e == cudaSuccess && check && GF.smem >= G.smem) e = gravity_ready(GF, gker_full);
     if (e != cudaSuccess) return e;
     if (A.force.fit) {
         // the fixed-node fits: the same table for every context, ordered on
@@ -642,11 +639,8 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
         e = cudaMemcpyToSymbolAsync(jb::c_fixed_fit, A.fit_host, sizeof(jb::JbFit), 0, cudaMemcpyHostToDevice, user);
         if (e != cudaSuccess) return e;
     }
-    // one CTA per SM (the table fills shared memory); each takes an equal
-    // share of the active slots, NT per thread
-    int gblocks = device_sm_count();
-    if (gblocks > A.n) gblocks = (int)A.n;
-    if (gblocks < 1) gblocks = 1;
+    // one CTA per SM (the table fills shared memory)
+    const int gctas = G.grid(A.n), gctas_full = GF.grid(A.n);
 
     // private stream ordered after the caller's stream (graphs need a
     // capturable stream)
@@ -692,20 +686,20 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
             timed(kKcPrep, [&] { pl_prep<M><<<blocks, kBlock, 0, st>>>(A, P, cur, s); });
             if (A.force.gravity_on)
                 timed(kKcGravity, [&] {
-                    gker<<<gblocks, gthreads, smem, st>>>(GT, gparts, P, cur, P.agrav, nullptr, nullptr);
+                    gravity_run(G, gker, gctas, st, GT, G.aux, P, cur, P.agrav, nullptr, nullptr);
                     if (sur) {
                         pl_earth_fixed<<<blocks, kBlock, 0, st>>>(P, cur);
                         launch_surrogate_stage(A.sur, &P.count[cur], A.n, P.ef, P.agrav, 1, P.cap, st);
                         if (check && s == 0) {
                             // the exact field of every evaluated row, then the verdicts
                             cudaMemsetAsync(P.fcount, 0, sizeof(int32_t), st);
-                            gker<<<gblocks, gthreads, smem_full, st>>>(A.sur.full, gparts_full, P, cur, P.agx,
-                                                                      nullptr, nullptr);
+                            gravity_run(GF, gker_full, gctas_full, st, A.sur.full, GF.aux, P, cur, P.agx, nullptr,
+                                        nullptr);
                             pl_sur_check<<<blocks, kBlock, 0, st>>>(P, cur, A.sur.check);
                         } else if (check) {
                             // the rows on the exact field for this step
-                            gker<<<gblocks, gthreads, smem_full, st>>>(A.sur.full, gparts_full, P, cur, P.agrav,
-                                                                      P.flist, P.fcount);
+                            gravity_run(GF, gker_full, gctas_full, st, A.sur.full, GF.aux, P, cur, P.agrav, P.flist,
+                                        P.fcount);
                         }
                     }
                 });

@@ -5,11 +5,12 @@
 //   k_propagate persistent one-trajectory-per-thread adaptive RK driver with
 //               Encke rectification, fed by a device work queue
 //
-// The gravity coefficient table is staged once per CTA into shared memory
-// (168 KB at degree 70) and read by warp-wide broadcasts.
+// The gravity coefficient table is staged per CTA into shared memory (146 KB
+// at degree 70) and read by warp-wide broadcasts.
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "launch.h"
@@ -18,16 +19,15 @@
 namespace bqp {
 
 // ----------------------------------------------------------------- kernels
-template <int NT>
-__global__ void __launch_bounds__(256, 1) k_gravity(GravTable T, int parts_max, int64_t n,
+template <int NT, int kForm>
+__global__ void __launch_bounds__(256, 1) k_gravity(const __grid_constant__ GravTable T, int aux, int64_t n,
                                                     const double* __restrict__ pos, double* __restrict__ acc,
                                                     int32_t* __restrict__ status) {
-    // rows are int-indexed inside a CTA: the launcher keeps each CTA's range
-    // below 2^31 by running chunks
-    const int64_t per_block = (n + gridDim.x - 1) / gridDim.x;
-    const int64_t c0 = (int64_t)blockIdx.x * per_block;
-    const int64_t c1 = c0 + per_block < n ? c0 + per_block : n;
-    if (c0 >= c1) return;  // uniform across the CTA
+    // rows are int-indexed inside a CTA or cluster: the launcher keeps its
+    // range below 2^31 by running chunks
+    int64_t per, c0, c1;
+    gravity_rows<kForm>(n, aux, &per, &c0, &c1);
+    if (c0 >= c1) return;  // uniform across the CTA and its cluster
     const double* p0 = pos + 3 * c0;
     double* a0 = acc + 3 * c0;
     int32_t* s0 = status ? status + c0 : nullptr;
@@ -44,9 +44,10 @@ __global__ void __launch_bounds__(256, 1) k_gravity(GravTable T, int parts_max, 
         z = ez;
         return true;
     };
-    auto store = [&](int i, const double* a, double x, double y, double z) {
+    auto store = [&](int i, const double* a) {
         // add the C00 point mass back: the full field of the reference's
         // spherical_gravity_impl_frame_packed (gravity.rs:2638-2675)
+        const double x = p0[3 * i], y = p0[3 * i + 1], z = p0[3 * i + 2];
         const double r2 = fma(x, x, fma(y, y, z * z));
         const double k = kMu / (r2 * sqrt(r2));
         a0[3 * i] = fma(-k, x, a[0]);
@@ -58,15 +59,15 @@ __global__ void __launch_bounds__(256, 1) k_gravity(GravTable T, int parts_max, 
         a0[3 * i] = a0[3 * i + 1] = a0[3 * i + 2] = NAN;
         if (s0) s0[i] = kWatchdog;
     };
-    gravity_cta<NT>(T, parts_max, (int)per_block, 0, (int)(c1 - c0), load, store, lost);
+    gravity_cta<NT, kForm>(T, aux, (int)per, 0, (int)(c1 - c0), load, store, lost);
 }
 
-__global__ void k_rhs(const double* __restrict__ gtab, int ncells, int use_smem, ForceParams fp,
+__global__ void k_rhs(const double* __restrict__ gtab, uint32_t tab_bytes, int use_smem, ForceParams fp,
                       int64_t n, const double* __restrict__ equ, const double* __restrict__ seg_t0,
                       const double* __restrict__ jd0, const double* __restrict__ t,
                       const double* __restrict__ delta, const double* __restrict__ ballistic,
                       double am0, double cd0, double* __restrict__ out) {
-    const double* tab = stage_table(gtab, ncells, use_smem != 0);
+    const double* tab = stage_table(gtab, tab_bytes, use_smem != 0);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         Encke R;
@@ -97,7 +98,7 @@ template <int M>
 __global__ void __launch_bounds__(256, 1) k_propagate(PropArgs A) {
     using T = Tab<M>;
     constexpr int S = T::S;
-    const double* tab = stage_table(A.gtab, A.ncells, A.use_smem != 0);
+    const double* tab = stage_table(A.gtab, A.tab_bytes, A.use_smem != 0);
     Encke R;
     R.tab = tab;
     R.fp = &A.force;
@@ -211,30 +212,23 @@ static int sm_count() {
 cudaError_t launch_gravity(const GravTable& T, int64_t n, const double* pos, double* acc, int32_t* status,
                            cudaStream_t st, int threads, int slots) {
     if (n <= 0) return cudaSuccess;
-    const int nt = slots == 1 || slots == 2 ? slots : 4;
-    auto ker = nt == 1 ? k_gravity<1> : (nt == 2 ? k_gravity<2> : k_gravity<4>);
-    if (threads <= 0 || threads > 256) threads = 256;
-    if (threads < 32) threads = 32;
-    threads = threads / 32 * 32;
-    int parts = kGravityPartsMax;
-    size_t smem = gravity_smem_bytes(T, threads, nt, parts);
-    if (smem > kSmemPerBlock) {
-        parts = 1;
-        smem = gravity_smem_bytes(T, threads, nt, parts);
-    }
-    cudaError_t e = cudaFuncSetAttribute(ker, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    GravLaunch G = gravity_launch(T, n, sm_count(), threads, slots);
+    auto of = [&](auto form) {
+        constexpr int F = decltype(form)::value;
+        return G.nt == 1 ? k_gravity<1, F> : G.nt == 2 ? k_gravity<2, F> : k_gravity<4, F>;
+    };
+    auto ker = G.form == kGravSplit     ? of(std::integral_constant<int, kGravSplit>())
+               : G.form == kGravCluster ? of(std::integral_constant<int, kGravCluster>())
+                                        : of(std::integral_constant<int, kGravPlain>());
+    cudaError_t e = gravity_ready(G, ker);
     if (e != cudaSuccess) return e;
-    // one CTA per SM; each takes an equal share of the rows.  Chunks of at
-    // most 2^30 rows keep a CTA's share int-indexed.
-    const int64_t grid_cap = (int64_t)sm_count();
+    // one CTA per SM; each (or each cluster) takes an equal share of the
+    // rows.  Chunks of at most 2^30 rows keep a share int-indexed.
     const int64_t chunk = (int64_t)1 << 30;
     for (int64_t off = 0; off < n; off += chunk) {
         const int64_t m = n - off < chunk ? n - off : chunk;
-        int64_t blocks = (m + 32 * nt - 1) / (32 * nt);
-        if (blocks > grid_cap) blocks = grid_cap;
-        ker<<<(unsigned)blocks, threads, smem, st>>>(T, parts, m, pos + 3 * off, acc + 3 * off,
-                                                     status ? status + off : nullptr);
-        e = cudaGetLastError();
+        e = gravity_run(G, ker, G.grid(m), st, T, G.aux, m, pos + 3 * off, acc + 3 * off,
+                        status ? status + off : nullptr);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -278,12 +272,12 @@ cudaError_t launch_jb_lookup(const jb::DriverTable& T, const double* jd, int64_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_rhs(const double* gtab, int ncells, int use_smem, const ForceParams& fp, int64_t n,
+cudaError_t launch_rhs(const double* gtab, uint32_t tab_bytes, int use_smem, const ForceParams& fp, int64_t n,
                        const double* equ, const double* seg_t0, const double* jd0, const double* t,
                        const double* delta, const double* ballistic, double am0, double cd0,
                        double* out, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const size_t smem = use_smem ? (size_t)ncells * kCellDoubles * sizeof(double) : 0;
+    const size_t smem = use_smem ? tab_bytes : 0;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -292,14 +286,14 @@ cudaError_t launch_rhs(const double* gtab, int ncells, int use_smem, const Force
     int64_t blocks = (n + threads - 1) / threads;
     const int64_t cap = (int64_t)sm_count();
     if (blocks > cap) blocks = cap;
-    k_rhs<<<(unsigned)blocks, threads, smem, st>>>(gtab, ncells, use_smem, fp, n, equ, seg_t0, jd0, t, delta,
+    k_rhs<<<(unsigned)blocks, threads, smem, st>>>(gtab, tab_bytes, use_smem, fp, n, equ, seg_t0, jd0, t, delta,
                                                    ballistic, am0, cd0, out);
     return cudaGetLastError();
 }
 
 template <int M>
 static cudaError_t launch_prop_m(const PropArgs& A, int threads, int blocks, cudaStream_t st) {
-    const size_t smem = A.use_smem ? (size_t)A.ncells * kCellDoubles * sizeof(double) : 0;
+    const size_t smem = A.use_smem ? A.tab_bytes : 0;
     cudaError_t e = cudaFuncSetAttribute(k_propagate<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(smem > 0 ? smem : 0));
     if (e != cudaSuccess) return e;
