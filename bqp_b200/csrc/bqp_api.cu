@@ -976,7 +976,8 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
         A.ecl = ctx->d_ecl;
     }
     if (ctx->cfg.engine == BQP_ENGINE_PIPELINE) {
-        const size_t need = pipeline_bytes(n);
+        const int iau = A.force.frame.mode == 1 ? 1 : 0;
+        const size_t need = pipeline_bytes(n, iau);
         if (need > ctx->pws_bytes) {
             if (ctx->d_pws) {
                 cudaStreamSynchronize(ctx->stream);
@@ -989,8 +990,7 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
             ctx->pws_bytes = need;
         }
         PipeBufs P{};
-        pipeline_carve(P, ctx->d_pws, n);
-        P.iau = A.force.frame.mode == 1 ? 1 : 0;
+        pipeline_carve(P, ctx->d_pws, n, iau);
         cudaError_t e = launch_pipeline(A, P, ctx->cfg.method, ctx->stream, ctx->cfg.max_kernel_seconds,
                                         ctx->cfg.gravity_threads, ctx->cfg.gravity_slots,
                                         ctx->profile ? &ctx->times : nullptr);

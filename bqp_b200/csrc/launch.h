@@ -64,19 +64,19 @@ struct PipeBufs {
     int32_t* count;       // [2] active counts
     double* k;            // [(S+1)][6][cap] stage derivatives
     double* sp;           // [6][cap] perturbed state of the stage (ECI)
-    double* sc;           // [2][cap] sin, cos of the GMST angle
-    double* fr;           // [12][cap] IAU frame: R (row-major) and ITRS angular velocity (GCRS)
-    int32_t iau;          // 1: the Earth-fixed frame is fr (IAU 2006/2000A), 0: sc (GMST)
-    double* sun;          // [3][cap] Sun position (ECI), drag only
+    // what a stage needs of its instant alone, formed for several stages at
+    // once: a ring of `ring` stages of [fields][cap] (StageTimes, pipeline.cu)
+    double* tq;
+    int32_t ring, fields;
+    int32_t iau;          // 1: the Earth-fixed frame is the IAU 2006/2000A one, 0: GMST
     double* part;         // [3][cap] third-body + Battin acceleration (ECI)
     double* agrav;        // [3][cap] gravity (Earth-fixed)
     double* adrag;        // [3][cap] drag (ECI)
-    double* jd;           // [cap]
     double* amcd;         // [2][cap]
     int32_t* skip;        // [cap] 1: stage derivative reused, no force call
     int32_t* bad;         // [cap] latched invalid-radius gravity error
     int32_t* dlist[2];    // drag work lists of the stage: 0 above ~510 km (sweep fits), 1 below
-    int32_t* dcount;      // [2]
+    int32_t* dcount;      // [ring][2]
     double* ef;           // [cap][3] Earth-fixed positions of the stage (surrogate gravity)
     // surrogate residual check (surrogate with a check only)
     double* agx;          // [3][cap] the exact field of the step's first stage
@@ -93,8 +93,8 @@ struct KernelTimes {
     int64_t launches[kKcCount];
 };
 
-size_t pipeline_bytes(int64_t cap);
-void pipeline_carve(PipeBufs& P, void* base, int64_t cap);
+size_t pipeline_bytes(int64_t cap, int iau);
+void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau);
 cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st,
                             double max_seconds, int gravity_threads, int gravity_slots,
                             KernelTimes* times = nullptr);

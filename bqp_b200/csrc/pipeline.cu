@@ -7,9 +7,11 @@
 // pass over three specialised kernels, and one controller kernel closes the
 // attempt:
 //
-//   pl_prep<M>(s)   finish stage s-1, form y_s = y + h sum a_sj k_j, the Encke
-//                   baseline (Kepler solve), Earth rotation, Sun/Moon third body
-//                   and Battin's term                       (latency / SFU bound)
+//   pl_times<M>     for several stages at once, what depends on a stage's
+//                   instant alone: Kepler baseline, Earth rotation, Sun, Moon
+//                                                           (FP64 latency bound)
+//   pl_prep<M>(s)   finish stage s-1, form y_s = y + h sum a_sj k_j, third body
+//                   and Battin's term                       (load latency bound)
 //   pl_gravity      normalised column recursion, table in shared memory
 //                                                           (FP64-FMA bound)
 //   pl_drag         JB2008 density and co-rotating drag     (transcendental bound)
@@ -22,6 +24,7 @@
 // and replayed; the host reads the active count between replays.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <cstdint>
 #include <vector>
@@ -71,32 +74,50 @@ __device__ __forceinline__ void append_active(int32_t* list, int32_t* count, int
     list[base + rank] = traj;
 }
 
+// What stage `st` needs of its instant, in the ring.
+struct StageTimes {
+    double* p;
+    int64_t cap;
+    __device__ __forceinline__ StageTimes(const PipeBufs& P, int st)
+        : p(P.tq + (size_t)(st % P.ring) * P.fields * P.cap), cap(P.cap) {}
+    __device__ __forceinline__ double& at(int field, int slot) const { return p[(size_t)field * cap + slot]; }
+    __device__ __forceinline__ double& baseline(int i, int slot) const { return at(i, slot); }
+    __device__ __forceinline__ double& sun(int i, int slot) const { return at(6 + i, slot); }
+    __device__ __forceinline__ double& moon(int i, int slot) const { return at(9 + i, slot); }
+    __device__ __forceinline__ double& jd(int slot) const { return at(12, slot); }
+    // GMST: sin, cos; IAU: R (row-major) and the ITRS angular velocity (GCRS)
+    __device__ __forceinline__ double& frame(int i, int slot) const { return at(13 + i, slot); }
+};
+constexpr int kTimesGmst = 15, kTimesIau = 25;
+
 // Sum of the stage-`st` force terms into K(st, 3..5).
 __device__ __forceinline__ void finish_stage(const PipeBufs& P, int st, int slot) {
+    const StageTimes T(P, st);
     const double gx = P.agrav[slot], gy = P.agrav[P.cap + slot], gz = P.agrav[2 * P.cap + slot];
     if (P.iau) {
         double r[9], g[3];
         const double gi[3] = {gx, gy, gz};
-        for (int e = 0; e < 9; ++e) r[e] = P.fr[(size_t)e * P.cap + slot];
+        for (int e = 0; e < 9; ++e) r[e] = T.frame(e, slot);
         ft::to_gcrs(r, gi, g);
         for (int i = 0; i < 3; ++i)
             K(P, st, 3 + i)[slot] = g[i] + P.adrag[(size_t)i * P.cap + slot] + P.part[(size_t)i * P.cap + slot];
         return;
     }
-    const double s = P.sc[slot], c = P.sc[P.cap + slot];
+    const double s = T.frame(0, slot), c = T.frame(1, slot);
     K(P, st, 3)[slot] = fma(c, gx, -s * gy) + P.adrag[slot] + P.part[slot];
     K(P, st, 4)[slot] = fma(s, gx, c * gy) + P.adrag[P.cap + slot] + P.part[P.cap + slot];
     K(P, st, 5)[slot] = gz + P.adrag[2 * P.cap + slot] + P.part[2 * P.cap + slot];
 }
 
-// An ECI vector of slot `slot` in the Earth-fixed frame of its stage.
-__device__ __forceinline__ void slot_to_itrs(const PipeBufs& P, int slot, const double* v, double* o) {
+// An ECI vector of slot `slot` in the Earth-fixed frame of stage T.
+__device__ __forceinline__ void slot_to_itrs(const PipeBufs& P, const StageTimes& T, int slot, const double* v,
+                                             double* o) {
     if (P.iau) {
         double r[9];
-        for (int e = 0; e < 9; ++e) r[e] = P.fr[(size_t)e * P.cap + slot];
+        for (int e = 0; e < 9; ++e) r[e] = T.frame(e, slot);
         ft::to_itrs(r, v, o);
     } else {
-        const double s = P.sc[slot], c = P.sc[P.cap + slot];
+        const double s = T.frame(0, slot), c = T.frame(1, slot);
         o[0] = fma(c, v[0], s * v[1]);
         o[1] = fma(-s, v[0], c * v[1]);
         o[2] = v[2];
@@ -124,10 +145,64 @@ __global__ void __launch_bounds__(kBlock) pl_init(PropArgs A, PipeBufs P) {
     append_active(P.idx[0], &P.count[0], (int32_t)traj, keep);
 }
 
+// -------------------------------------------------------------------- times
+// Stages st0 .. st0 + gridDim.y - 1 of the current attempt, one stage of one
+// row a thread.  st == S is the dense-output stage of the sampled non-FSAL
+// path: f(t_next, y_next) evaluated before the controller decides (the
+// reference evaluates it after an accept).
+//
+// Everything here is known when the attempt begins, so the stages' long FP64
+// chains (the Kepler solve, the Sun and Moon series, the frame) run side by
+// side once an attempt instead of one after the other before each stage's
+// force.
+template <int M>
+__global__ void __launch_bounds__(kBlock) pl_times(PropArgs A, PipeBufs P, int cur, int st0) {
+    using T = Tab<M>;
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x, st = st0 + blockIdx.y;
+    if (blockIdx.x == 0 && threadIdx.x < 2) P.dcount[2 * (st % P.ring) + threadIdx.x] = 0;
+    if (slot >= P.count[cur]) return;
+    const TrajState& s = P.st[P.idx[cur][slot]];
+    if (st == 0 && (s.flags & kHaveK1)) return;
+    const StageTimes Q(P, st);
+    const double ts = st < T::S ? s.t + T::c(st) * s.hs : next_time(s);
+    double rs[6];
+    baseline_state(baseline_new(s.cur), ts - s.ct0, rs);
+    for (int i = 0; i < 6; ++i) Q.baseline(i, slot) = rs[i];
+    const double jd = utc_jd_at(s.jd0, ts);
+    Q.jd(slot) = jd;
+    const ForceParams& fp = A.force;
+    if (P.iau) {
+        // the IAU 2006/2000A rotation of the stage's instant (rhs.rs:3113-3174);
+        // NaN where it has none
+        ft::FrameRot F;
+        if ((fp.gravity_on || fp.drag) && !frame_rot(fp.frame, s.tai0 + ts, F)) {
+            for (int e = 0; e < 9; ++e) F.r[e] = NAN;
+            F.w[0] = F.w[1] = F.w[2] = NAN;
+        } else if (!(fp.gravity_on || fp.drag)) {
+            for (int e = 0; e < 9; ++e) F.r[e] = (e % 4 == 0) ? 1.0 : 0.0;
+            F.w[0] = F.w[1] = F.w[2] = 0.0;
+        }
+        for (int e = 0; e < 9; ++e) Q.frame(e, slot) = F.r[e];
+        for (int e = 0; e < 3; ++e) Q.frame(9 + e, slot) = F.w[e];
+    } else {
+        double sn = 0.0, cs = 1.0;
+        if (fp.gravity_on || fp.drag) sincos(gmst_rad(jd), &sn, &cs);
+        Q.frame(0, slot) = sn;
+        Q.frame(1, slot) = cs;
+    }
+    if (fp.sun || (fp.drag && s.cd != 0.0 && s.am != 0.0) || s.side >= 0) {
+        double sun[3];
+        sun_at(fp.eph_sun, jd, sun);
+        for (int i = 0; i < 3; ++i) Q.sun(i, slot) = sun[i];
+    }
+    if (fp.moon) {
+        double moon[3];
+        moon_at(fp.eph_moon, jd, moon);
+        for (int i = 0; i < 3; ++i) Q.moon(i, slot) = moon[i];
+    }
+}
+
 // --------------------------------------------------------------------- prep
-// Stage `st` of the current attempt.  st == S is the dense-output stage of
-// the sampled non-FSAL path: f(t_next, y_next) evaluated before the
-// controller decides (the reference evaluates it after an accept).
 template <int M>
 __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cur, int st) {
     using T = Tab<M>;
@@ -150,7 +225,6 @@ __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cu
     // stage state
     double yt[6];
     for (int i = 0; i < 6; ++i) yt[i] = s.y[i];
-    double ts;
     if (st < T::S) {
 #pragma unroll 1
         for (int j = 0; j < st; ++j) {
@@ -158,7 +232,6 @@ __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cu
             if (a != 0.0)
                 for (int i = 0; i < 6; ++i) yt[i] = fma(K(P, j, i)[slot], a, yt[i]);
         }
-        ts = s.t + T::c(st) * s.hs;
     } else {
         // y_next exactly as rk_combine forms it
 #pragma unroll 1
@@ -167,54 +240,32 @@ __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cu
             if (b != 0.0)
                 for (int i = 0; i < 6; ++i) yt[i] = fma(K(P, j, i)[slot], b, yt[i]);
         }
-        ts = next_time(s);
     }
-    double rs[6];
-    baseline_state(baseline_new(s.cur), ts - s.ct0, rs);
-    double sp[6];
+    const StageTimes Q(P, st);
+    double rs[6], sp[6];
     for (int i = 0; i < 6; ++i) {
+        rs[i] = Q.baseline(i, slot);
         sp[i] = rs[i] + yt[i];
         P.sp[(size_t)i * P.cap + slot] = sp[i];
     }
     for (int i = 0; i < 3; ++i) K(P, st, i)[slot] = yt[3 + i];
-    const double jd = utc_jd_at(s.jd0, ts);
     const ForceParams& fp = A.force;
-    if (P.iau) {
-        // the IAU 2006/2000A rotation of the stage's instant (rhs.rs:3113-3174)
-        ft::FrameRot F;
-        if ((fp.gravity_on || fp.drag) && !frame_rot(fp.frame, s.tai0 + ts, F)) {
-            P.bad[slot] = 3;
-            for (int e = 0; e < 9; ++e) F.r[e] = NAN;
-            F.w[0] = F.w[1] = F.w[2] = NAN;
-        } else if (!(fp.gravity_on || fp.drag)) {
-            for (int e = 0; e < 9; ++e) F.r[e] = (e % 4 == 0) ? 1.0 : 0.0;
-            F.w[0] = F.w[1] = F.w[2] = 0.0;
-        }
-        for (int e = 0; e < 9; ++e) P.fr[(size_t)e * P.cap + slot] = F.r[e];
-        for (int e = 0; e < 3; ++e) P.fr[(size_t)(9 + e) * P.cap + slot] = F.w[e];
-    } else {
-        double sn = 0.0, cs = 1.0;
-        if (fp.gravity_on || fp.drag) sincos(gmst_rad(jd), &sn, &cs);
-        P.sc[slot] = sn;
-        P.sc[P.cap + slot] = cs;
-    }
+    if (P.iau && (fp.gravity_on || fp.drag) && isnan(Q.frame(0, slot))) P.bad[slot] = 3;
     double acc[3] = {0.0, 0.0, 0.0};
     double sun[3];
     const bool need_sun = fp.sun || (fp.drag && s.cd != 0.0 && s.am != 0.0) || s.side >= 0;
-    if (need_sun) sun_at(fp.eph_sun, jd, sun);
+    if (need_sun)
+        for (int i = 0; i < 3; ++i) sun[i] = Q.sun(i, slot);
     if (s.side >= 0) srp_accel(sp, sun, fp.p_sun, fp.cr, s.am, s.side, acc);  // on the leg's fixed side
     if (fp.sun) third_body(sp, sun, fp.mu_sun, acc);
     if (fp.moon) {
-        double moon[3];
-        moon_at(fp.eph_moon, jd, moon);
+        const double moon[3] = {Q.moon(0, slot), Q.moon(1, slot), Q.moon(2, slot)};
         third_body(sp, moon, fp.mu_moon, acc);
     }
     const double r2 = fma(sp[0], sp[0], fma(sp[1], sp[1], sp[2] * sp[2]));
     battin(rs, yt, r2, sqrt(r2), acc);
     for (int i = 0; i < 3; ++i) P.part[(size_t)i * P.cap + slot] = acc[i];
     if (fp.drag) {
-        for (int i = 0; i < 3; ++i) P.sun[(size_t)i * P.cap + slot] = sun[i];
-        P.jd[slot] = jd;
         P.amcd[slot] = s.am;
         P.amcd[P.cap + slot] = s.cd;
         // drag work list: states above ~510 km take the sweep fits (cheap),
@@ -228,7 +279,7 @@ __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cu
                 const int lane = threadIdx.x & 31;
                 const int leader = __ffs(mm) - 1;
                 int base = 0;
-                if (lane == leader) base = atomicAdd(&P.dcount[c], __popc(mm));
+                if (lane == leader) base = atomicAdd(&P.dcount[2 * (st % P.ring) + c], __popc(mm));
                 base = __shfl_sync(mm, base, leader);
                 P.dlist[c][base + __popc(mm & ((1u << lane) - 1u))] = slot;
             }
@@ -247,17 +298,19 @@ __global__ void __launch_bounds__(kBlock) pl_prep(PropArgs A, PipeBufs P, int cu
 // list[0 .. *list_count) instead of the active slots 0 .. count.
 template <int NT, int kForm>
 __global__ void __launch_bounds__(256, 1) pl_gravity(const __grid_constant__ GravTable T, int aux, PipeBufs P, int cur,
-                                                     double* out, const int32_t* list, const int32_t* list_count) {
+                                                     int st, double* out, const int32_t* list,
+                                                     const int32_t* list_count) {
     int64_t per, c0, c1;
     gravity_rows<kForm>(list ? *list_count : P.count[cur], aux, &per, &c0, &c1);
     const int b0 = (int)c0, b1 = (int)c1;
+    const StageTimes Q(P, st);
     if (b0 >= b1) return;  // uniform across the CTA and its cluster
     auto load = [&](int row, double& x, double& y, double& z) -> bool {
         const int sl = list ? list[row] : row;
         if (P.skip[sl]) return false;
         const double e[3] = {P.sp[sl], P.sp[P.cap + sl], P.sp[2 * P.cap + sl]};
         double q[3];
-        slot_to_itrs(P, sl, e, q);
+        slot_to_itrs(P, Q, sl, e, q);
         const double r2 = fma(q[0], q[0], fma(q[1], q[1], q[2] * q[2]));
         if (!(isfinite(r2) && r2 > 0.0)) {
             if (!P.bad[sl]) P.bad[sl] = 1;
@@ -283,7 +336,7 @@ __global__ void __launch_bounds__(256, 1) pl_gravity(const __grid_constant__ Gra
     gravity_cta<NT, kForm>(T, aux, (int)per, b0, b1, load, store, lost);
 }
 
-using GravKernel = void (*)(const GravTable, int, PipeBufs, int, double*, const int32_t*, const int32_t*);
+using GravKernel = void (*)(const GravTable, int, PipeBufs, int, int, double*, const int32_t*, const int32_t*);
 
 template <int F>
 static GravKernel pl_gravity_form(int nt) {
@@ -298,11 +351,11 @@ static GravKernel pl_gravity_of(const GravLaunch& G) {
 
 // Earth-fixed positions of the stage's active slots, [slot][3] (the
 // surrogate's input)
-__global__ void __launch_bounds__(kBlock) pl_earth_fixed(PipeBufs P, int cur) {
+__global__ void __launch_bounds__(kBlock) pl_earth_fixed(PipeBufs P, int cur, int st) {
     const int sl = blockIdx.x * blockDim.x + threadIdx.x;
     if (sl >= P.count[cur]) return;
     const double e[3] = {P.sp[sl], P.sp[P.cap + sl], P.sp[2 * P.cap + sl]};
-    slot_to_itrs(P, sl, e, P.ef + 3 * (size_t)sl);
+    slot_to_itrs(P, StageTimes(P, st), sl, e, P.ef + 3 * (size_t)sl);
 }
 
 // ------------------------------------------------------- surrogate check
@@ -345,12 +398,12 @@ __global__ void __launch_bounds__(kBlock) pl_sur_check(PipeBufs P, int cur, doub
 // so that a stage's states are resident together in as few waves as the
 // register budget allows.
 template <int L, bool kCoarse = false>
-__device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs& P, int list, int block) {
+__device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs& P, int st, int list, int block) {
     const int gt = block * blockDim.x + threadIdx.x;
     const int item = gt / L;
     const int q = gt % L;
     const unsigned gmask = ((1u << L) - 1u) << ((threadIdx.x & 31) & ~(L - 1));
-    if (item >= P.dcount[list]) return;  // uniform across the group
+    if (item >= P.dcount[2 * (st % P.ring) + list]) return;  // uniform across the group
     const int slot = P.dlist[list][item];
     double sp[6];
     for (int i = 0; i < 6; ++i) sp[i] = P.sp[(size_t)i * P.cap + slot];
@@ -358,10 +411,12 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
     double a[3] = {0.0, 0.0, 0.0};
     if (cd != 0.0 && am != 0.0) {
         // JB2008 adapter (rhs.rs:3551-3776), as Encke::density_at
-        const double sun[3] = {P.sun[slot], P.sun[P.cap + slot], P.sun[2 * P.cap + slot]};
+        const StageTimes Q(P, st);
+        const double sun[3] = {Q.sun(0, slot), Q.sun(1, slot), Q.sun(2, slot)};
+        const double jd = Q.jd(slot);
         double pi[3], si[3];
-        slot_to_itrs(P, slot, sp, pi);
-        slot_to_itrs(P, slot, sun, si);
+        slot_to_itrs(P, Q, slot, sp, pi);
+        slot_to_itrs(P, Q, slot, sun, si);
         const double sun_r = sqrt(fma(si[0], si[0], fma(si[1], si[1], si[2] * si[2])));
         const double sat_r = sqrt(fma(pi[0], pi[0], fma(pi[1], pi[1], pi[2] * pi[2])));
         double rho;
@@ -376,14 +431,14 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
             // fixed-node fits from constant memory (fp.fit holds the same numbers);
             // no drivers at this instant -> NaN density (rhs.rs:3560-3571), the
             // same verdict on every lane of the group
-            if (fp.dtab.n_solar > 0 && !jb::lookup_drivers(fp.dtab, P.jd[slot], &dr))
+            if (fp.dtab.n_solar > 0 && !jb::lookup_drivers(fp.dtab, jd, &dr))
                 rho = NAN;
             else if (kCoarse && fp.drag_fp32)
-                rho = jb::density_coarse_r<float>(P.jd[slot] - 2400000.5, dec, ha, lat, alt_m, dr, fp.atm_model);
+                rho = jb::density_coarse_r<float>(jd - 2400000.5, dec, ha, lat, alt_m, dr, fp.atm_model);
             else if (kCoarse)
-                rho = jb::density_coarse(P.jd[slot] - 2400000.5, dec, ha, lat, alt_m, dr, fp.atm_model);
+                rho = jb::density_coarse(jd - 2400000.5, dec, ha, lat, alt_m, dr, fp.atm_model);
             else
-                rho = jb::density_group<L>(P.jd[slot] - 2400000.5, dec, ha, lat, alt_m, dr, q, gmask,
+                rho = jb::density_group<L>(jd - 2400000.5, dec, ha, lat, alt_m, dr, q, gmask,
                                            fp.fit != nullptr, fp.fit2);
             if (!(rho > 0.0) || !isfinite(rho)) rho = NAN;
             else if (alt_m > 2500.0e3) rho = fmin(rho, 1.0e-19);
@@ -395,7 +450,8 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
             if (P.iau) {
                 // atmosphere co-rotating with the resolved frame (rhs.rs:1134-1139)
                 double w[3];
-                for (int e = 0; e < 3; ++e) w[e] = P.fr[(size_t)(9 + e) * P.cap + slot];
+                const StageTimes Q(P, st);
+                for (int e = 0; e < 3; ++e) w[e] = Q.frame(9 + e, slot);
                 vr0 = (sp[3] - (w[1] * sp[2] - w[2] * sp[1])) * 1000.0;
                 vr1 = (sp[4] - (w[2] * sp[0] - w[0] * sp[2])) * 1000.0;
                 vr2 = (sp[5] - (w[0] * sp[1] - w[1] * sp[0])) * 1000.0;
@@ -419,16 +475,16 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
 }
 
 template <int LH, int LL>
-__global__ void __launch_bounds__(kBlock, BQP_DRAG_MIN_BLOCKS) pl_drag(ForceParams fp, PipeBufs P, int nb_hi) {
-    if ((int)blockIdx.x < nb_hi) drag_rows<LH>(fp, P, 0, blockIdx.x);
-    else drag_rows<LL>(fp, P, 1, blockIdx.x - nb_hi);
+__global__ void __launch_bounds__(kBlock, BQP_DRAG_MIN_BLOCKS) pl_drag(ForceParams fp, PipeBufs P, int st, int nb_hi) {
+    if ((int)blockIdx.x < nb_hi) drag_rows<LH>(fp, P, st, 0, blockIdx.x);
+    else drag_rows<LL>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
 // The coarse profiles (atm_model 5-7): a short chain per state, one lane
 // each, both altitude lists in one launch.
-__global__ void __launch_bounds__(kBlock) pl_drag_coarse(ForceParams fp, PipeBufs P, int nb_hi) {
-    if ((int)blockIdx.x < nb_hi) drag_rows<1, true>(fp, P, 0, blockIdx.x);
-    else drag_rows<1, true>(fp, P, 1, blockIdx.x - nb_hi);
+__global__ void __launch_bounds__(kBlock) pl_drag_coarse(ForceParams fp, PipeBufs P, int st, int nb_hi) {
+    if ((int)blockIdx.x < nb_hi) drag_rows<1, true>(fp, P, st, 0, blockIdx.x);
+    else drag_rows<1, true>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
 // ------------------------------------------------------------------ control
@@ -564,13 +620,23 @@ __global__ void __launch_bounds__(kBlock) pl_abort(PropArgs A, PipeBufs P, int c
 }
 
 // ------------------------------------------------------------------- host
-size_t pipeline_bytes(int64_t cap) {
-    PipeBufs P{};
-    pipeline_carve(P, nullptr, cap);
-    return (size_t)(uintptr_t)P.dcount + 2 * sizeof(int32_t) + 256;
+// Stages whose instants are prepared at once: as many as leave their
+// quantities (200 B a row and stage, 120 in the GMST frame) in L2 beside what
+// the stages themselves touch, at least one.  The ring has one more, the
+// stage before a group, which is finished after the group is prepared.
+static int times_group(int64_t cap, int fields) {
+    const int64_t one = cap * fields * 8;
+    const int64_t g = one > 0 ? ((int64_t)96 << 20) / one : kStageBufs;
+    return (int)(g < 1 ? 1 : (g > kStageBufs ? kStageBufs : g));
 }
 
-void pipeline_carve(PipeBufs& P, void* base, int64_t cap) {
+size_t pipeline_bytes(int64_t cap, int iau) {
+    PipeBufs P{};
+    pipeline_carve(P, nullptr, cap, iau);
+    return (size_t)(uintptr_t)P.dcount + 2 * (size_t)P.ring * sizeof(int32_t) + 256;
+}
+
+void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
         off = (off + 255) & ~(size_t)255;
@@ -586,13 +652,13 @@ void pipeline_carve(PipeBufs& P, void* base, int64_t cap) {
     P.count = (int32_t*)take(2 * 4);
     P.k = (double*)take((size_t)kStageBufs * 6 * c * 8);
     P.sp = (double*)take(6 * c * 8);
-    P.sc = (double*)take(2 * c * 8);
-    P.fr = (double*)take(12 * c * 8);
-    P.sun = (double*)take(3 * c * 8);
+    P.iau = iau;
+    P.fields = iau ? kTimesIau : kTimesGmst;
+    P.ring = times_group(cap, P.fields) + 1;
+    P.tq = (double*)take((size_t)P.ring * P.fields * c * 8);
     P.part = (double*)take(3 * c * 8);
     P.agrav = (double*)take(3 * c * 8);
     P.adrag = (double*)take(3 * c * 8);
-    P.jd = (double*)take(c * 8);
     P.amcd = (double*)take(2 * c * 8);
     P.skip = (int32_t*)take(c * 4);
     P.bad = (int32_t*)take(c * 4);
@@ -603,7 +669,7 @@ void pipeline_carve(PipeBufs& P, void* base, int64_t cap) {
     P.fall = (int32_t*)take(c * 4);
     P.flist = (int32_t*)take(c * 4);
     P.fcount = (int32_t*)take(4);
-    P.dcount = (int32_t*)take(2 * 4);  // last: pipeline_bytes measures up to it
+    P.dcount = (int32_t*)take(2 * (size_t)P.ring * 4);  // last: pipeline_bytes measures up to it
 }
 
 template <int M>
@@ -614,6 +680,8 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     // the eclipse coordinator's Hermite scan
     const bool dense = (A.out_mode != kOutFinalEci || A.force.srp) && !T::FSAL;
     const int stages = T::S + (dense ? 1 : 0);
+    // equal groups of at most P.ring - 1 stages
+    const int groups = (stages + P.ring - 2) / (P.ring - 1), group = (stages + groups - 1) / groups;
     const int blocks = (int)((A.n + kBlock - 1) / kBlock);
     constexpr int kLanesHigh = BQP_DRAG_LANES_HIGH, kLanesLow = BQP_DRAG_LANES_LOW;
     const int dblocks_hi = (int)((A.n * kLanesHigh + kBlock - 1) / kBlock);
@@ -682,23 +750,26 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     // one graph = two attempts (active list 0 -> 1 -> 0)
     auto enqueue_attempt = [&](int cur, int timed_out) {
         for (int s = 0; s < stages; ++s) {
-            if (A.force.drag) cudaMemsetAsync(P.dcount, 0, 2 * sizeof(int32_t), st);
-            timed(kKcPrep, [&] { pl_prep<M><<<blocks, kBlock, 0, st>>>(A, P, cur, s); });
+            timed(kKcPrep, [&] {
+                if (s % group == 0)
+                    pl_times<M><<<dim3(blocks, std::min(group, stages - s)), kBlock, 0, st>>>(A, P, cur, s);
+                pl_prep<M><<<blocks, kBlock, 0, st>>>(A, P, cur, s);
+            });
             if (A.force.gravity_on)
                 timed(kKcGravity, [&] {
-                    gravity_run(G, gker, gctas, st, GT, G.aux, P, cur, P.agrav, nullptr, nullptr);
+                    gravity_run(G, gker, gctas, st, GT, G.aux, P, cur, s, P.agrav, nullptr, nullptr);
                     if (sur) {
-                        pl_earth_fixed<<<blocks, kBlock, 0, st>>>(P, cur);
+                        pl_earth_fixed<<<blocks, kBlock, 0, st>>>(P, cur, s);
                         launch_surrogate_stage(A.sur, &P.count[cur], A.n, P.ef, P.agrav, 1, P.cap, st);
                         if (check && s == 0) {
                             // the exact field of every evaluated row, then the verdicts
                             cudaMemsetAsync(P.fcount, 0, sizeof(int32_t), st);
-                            gravity_run(GF, gker_full, gctas_full, st, A.sur.full, GF.aux, P, cur, P.agx, nullptr,
+                            gravity_run(GF, gker_full, gctas_full, st, A.sur.full, GF.aux, P, cur, s, P.agx, nullptr,
                                         nullptr);
                             pl_sur_check<<<blocks, kBlock, 0, st>>>(P, cur, A.sur.check);
                         } else if (check) {
                             // the rows on the exact field for this step
-                            gravity_run(GF, gker_full, gctas_full, st, A.sur.full, GF.aux, P, cur, P.agrav, P.flist,
+                            gravity_run(GF, gker_full, gctas_full, st, A.sur.full, GF.aux, P, cur, s, P.agrav, P.flist,
                                         P.fcount);
                         }
                     }
@@ -706,10 +777,10 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
             if (A.force.drag)
                 timed(kKcDrag, [&] {
                     if (A.force.atm_model == 4)
-                        pl_drag<kLanesHigh, kLanesLow><<<dblocks_hi + dblocks_lo, kBlock, 0, st>>>(A.force, P,
-                                                                                                 dblocks_hi);
+                        pl_drag<kLanesHigh, kLanesLow>
+                            <<<dblocks_hi + dblocks_lo, kBlock, 0, st>>>(A.force, P, s, dblocks_hi);
                     else
-                        pl_drag_coarse<<<2 * blocks, kBlock, 0, st>>>(A.force, P, blocks);
+                        pl_drag_coarse<<<2 * blocks, kBlock, 0, st>>>(A.force, P, s, blocks);
                 });
         }
         timed(kKcControl, [&] { pl_control<M><<<blocks, kBlock, 0, st>>>(A, P, cur, dense ? 1 : 0, timed_out); });
