@@ -666,6 +666,7 @@ ForceParams force_params(const bqp_ctx* ctx) {
     // the sweep fits replace the exact model's quadrature only
     fp.fit = (c.drag_quadrature || !fp.drag || fp.atm_model != 4) ? nullptr : ctx->d_fit;
     fp.fit2 = fp.fit ? ctx->d_fit2 : nullptr;
+    if (fp.drag) fp.plan = fp.drag_fp32 ? jb::coarse_plan<float>(fp.atm_model) : jb::coarse_plan<double>(fp.atm_model);
     fp.frame = ctx->ftab;
     return fp;
 }
@@ -977,7 +978,7 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
     }
     if (ctx->cfg.engine == BQP_ENGINE_PIPELINE) {
         const int iau = A.force.frame.mode == 1 ? 1 : 0;
-        const size_t need = pipeline_bytes(n, iau);
+        const size_t need = pipeline_bytes(n, iau, A.force.drag);
         if (need > ctx->pws_bytes) {
             if (ctx->d_pws) {
                 cudaStreamSynchronize(ctx->stream);
@@ -990,7 +991,7 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
             ctx->pws_bytes = need;
         }
         PipeBufs P{};
-        pipeline_carve(P, ctx->d_pws, n, iau);
+        pipeline_carve(P, ctx->d_pws, n, iau, A.force.drag);
         cudaError_t e = launch_pipeline(A, P, ctx->cfg.method, ctx->stream, ctx->cfg.max_kernel_seconds,
                                         ctx->cfg.gravity_threads, ctx->cfg.gravity_slots,
                                         ctx->profile ? &ctx->times : nullptr);

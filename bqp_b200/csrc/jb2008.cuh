@@ -725,6 +725,70 @@ BQP_HD SweepR<R> boole_sweep_r(R z, R zend_start, R zr, int n, R ain, bool with_
     return s;
 }
 
+// What the model needs of the instant and the drivers alone: the solar part
+// of the exospheric temperature, the phase of the seasonal-latitudinal term
+// and the semiannual term's function of the day (NaN where the day is out of
+// range).  `coarse` picks the profiles' order of operations.
+template <class R>
+struct EpochR {
+    R tsubc, sinphi, gtz;
+};
+template <class R>
+BQP_HD EpochR<R> epoch_terms(double mjd, const Drivers& din, bool coarse) {
+    const R f10 = (R)din.f10, f10b = (R)din.f10b, s10 = (R)din.s10, s10b = (R)din.s10b, m10 = (R)din.m10,
+            m10b = (R)din.m10b, y10 = (R)din.y10, y10b = (R)din.y10b;
+    EpochR<R> E;
+    const R fn = rm::fmin(rm::pow(f10b / (R)240.0, (R)0.25), (R)1.0);
+    const R fsb = f10b * fn + s10b * ((R)1.0 - fn);
+    E.tsubc = (R)392.4 + (R)3.227 * fsb + (R)0.298 * (f10 - f10b) + (R)2.259 * (s10 - s10b) +
+              (R)0.312 * (m10 - m10b) + (R)0.178 * (y10 - y10b);
+    const double years = (mjd - 36204.0) / 365.2422;
+    double capphi = years - ::trunc(years);
+    if (capphi == 0.0) capphi = ::copysign(0.0, years);
+    E.sinphi = rm::sin((R)(kTwoPi * capphi + 1.72));
+    bool ok = true;
+    const double day = day_of_year(mjd, &ok);
+    R gtm[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) gtm[i] = (R)JBT(kGtm)[i];
+    const R fg = f10b - (R)0.75 * s10b - (R)0.37 * m10b;
+    R s1, c1;
+    rm::sincos((R)(kTwoPi * (day - 1.0) / 365.0), &s1, &c1);
+    const R s2 = (R)2.0 * s1 * c1, c2 = c1 * c1 - s1 * s1;
+    if (coarse)
+        E.gtz = gtm[0] + gtm[1] * s1 + gtm[2] * c1 + gtm[3] * s2 + gtm[4] * c2 +
+                fg * (gtm[5] + gtm[6] * s1 + gtm[7] * c1 + gtm[8] * s2 + gtm[9] * c2);
+    else
+        E.gtz = gtm[0] + gtm[1] * s1 + gtm[2] * c1 + gtm[3] * s2 + gtm[4] * c2 + gtm[5] * fg + gtm[6] * fg * s1 +
+                gtm[7] * fg * c1 + gtm[8] * fg * s2 + gtm[9] * fg * c2;
+    if (!ok) E.gtz = (R)NAN;
+    return E;
+}
+
+// The drivers' and the instant's part of the input checks.
+BQP_HD bool drivers_valid(double mjd, const Drivers& d) {
+    return isfinite(mjd) && isfinite(d.f10) && isfinite(d.f10b) && isfinite(d.s10) && isfinite(d.s10b) &&
+           isfinite(d.m10) && isfinite(d.m10b) && isfinite(d.y10) && isfinite(d.y10b) && isfinite(d.dtc) &&
+           !(d.f10 <= 0.0 || d.f10b <= 0.0 || d.s10 <= 0.0 || d.s10b <= 0.0 || d.m10 <= 0.0 || d.m10b <= 0.0 ||
+             d.y10 <= 0.0 || d.y10b <= 0.0);
+}
+
+// The state's part of them.
+BQP_HD bool geometry_valid(double sun_dec, double hour_angle, double lat, double alt_m) {
+    return isfinite(sun_dec) && isfinite(hour_angle) && isfinite(lat) && isfinite(alt_m) && alt_m >= 90000.0 &&
+           sun_dec >= -kPi / 2 && sun_dec <= kPi / 2 && lat >= -kPi / 2 && lat <= kPi / 2;
+}
+
+// Model 7's two fixed plans: where their walks end.  Inside the fit domain
+// their sums, and all else that depends on the temperatures, come from the
+// series, so what the walk would leave besides depends on nothing: the last
+// node and interval end of the 90-105 km plan with mbar and g there, and of
+// the 105-500 km plan.  Formed once on the host (coarse_plan).
+struct CoarsePlan {
+    double low_z, low_zend, low_mb, low_gravl, mid_z, mid_zend;
+    int32_t valid, pad;
+};
+
 // As density(), for atm_model 5, 6 or 7, in R after the input checks.  FP64:
 // the reference's arithmetic.  FP32: the split form's density; its relative
 // error (~1e-6: the exponents reach ~45) moves the drag acceleration by
@@ -732,32 +796,16 @@ BQP_HD SweepR<R> boole_sweep_r(R z, R zend_start, R zr, int n, R ain, bool with_
 // inside FP32's range.  The epoch terms (fractional year, day of year) are
 // kept in FP64, since an MJD does not fit FP32.
 template <class R>
-BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, double lat_in, double alt_m,
-                               const Drivers& din, int model) {
+BQP_HD double density_coarse_core(const EpochR<R>& E, double sun_dec, double hour_angle, double lat_in, double alt_m,
+                                  const Drivers& din, int model, const CoarsePlan* plan) {
     const R step_lower = (R)0.040, step_middle = model == 5 ? (R)0.100 : (R)0.300;
     const R step_upper = model == 5 ? (R)0.300 : (R)0.700;
     const bool v7 = model == 7;
-    if (!isfinite(mjd) || !isfinite(sun_dec) || !isfinite(hour_angle) || !isfinite(lat_in) ||
-        !isfinite(alt_m) || !isfinite(din.f10) || !isfinite(din.f10b) || !isfinite(din.s10) ||
-        !isfinite(din.s10b) || !isfinite(din.m10) || !isfinite(din.m10b) || !isfinite(din.y10) ||
-        !isfinite(din.y10b) || !isfinite(din.dtc))
-        return kErrNonFinite;
-    if (alt_m < 90000.0) return kErrAltitude;
-    if (!(sun_dec >= -kPi / 2 && sun_dec <= kPi / 2) || !(lat_in >= -kPi / 2 && lat_in <= kPi / 2))
-        return kErrAngle;
-    if (din.f10 <= 0.0 || din.f10b <= 0.0 || din.s10 <= 0.0 || din.s10b <= 0.0 || din.m10 <= 0.0 ||
-        din.m10b <= 0.0 || din.y10 <= 0.0 || din.y10b <= 0.0)
-        return kErrIndex;
     const R alt = (R)(alt_m / 1000.0);
     const R lat = (R)lat_in, sdec = (R)sun_dec;
-    const R f10 = (R)din.f10, f10b = (R)din.f10b, s10 = (R)din.s10, s10b = (R)din.s10b, m10 = (R)din.m10,
-            m10b = (R)din.m10b, y10 = (R)din.y10, y10b = (R)din.y10b, dtc_k = (R)din.dtc;
+    const R f10 = (R)din.f10, f10b = (R)din.f10b, s10b = (R)din.s10b, m10b = (R)din.m10b, dtc_k = (R)din.dtc;
     const R pi = (R)kPi, two_pi = (R)kTwoPi;
     // exospheric temperature and profile, as density()
-    const R fn = rm::fmin(rm::pow(f10b / (R)240.0, (R)0.25), (R)1.0);
-    const R fsb = f10b * fn + s10b * ((R)1.0 - fn);
-    const R tsubc = (R)392.4 + (R)3.227 * fsb + (R)0.298 * (f10 - f10b) + (R)2.259 * (s10 - s10b) +
-                    (R)0.312 * (m10 - m10b) + (R)0.178 * (y10 - y10b);
     const R eta = (R)0.5 * rm::fabs(lat - sdec);
     const R theta = (R)0.5 * rm::fabs(lat + sdec);
     R h = (R)hour_angle;
@@ -780,7 +828,7 @@ BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, do
     const R sin_theta = sn * sn * rm::sqrt(sn);
     const R cos_tau = rm::fabs(rm::cos((R)0.5 * tau));
     const R df = sin_theta + (cos_eta - sin_theta) * cos_tau * cos_tau * cos_tau;
-    const R tsubl = tsubc * ((R)1.0 + (R)0.31 * df);
+    const R tsubl = E.tsubc * ((R)1.0 + (R)0.31 * df);
     const R tinf = tsubl + dtc_k + dtc_correction_r(f10, st_hour, clat, alt);
     const R tsubx = (R)444.3807 + (R)0.02385 * tinf - (R)392.8292 * rm::exp((R)-0.0021357 * tinf);
     const R gsubx = (R)0.054285714 * (tsubx - (R)183.0);
@@ -799,10 +847,21 @@ BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, do
     const R mb1 = mbar_r(z1);
     const R tloc1 = local_temp_r(z1, tc);
     const bool lower_planned = alt >= (R)105.0;
-    R al = rm::log(rm::fmin(alt, (R)105.0) / z1);
-    int n = coarse_panels(al / step_lower);
-    if (n == 0) return kErrDomain;
-    SweepR<R> lo = boole_sweep_r(z1, z1, rm::exp(al / (R)n), n, mb1 * grav_r(z1) / tloc1, true, tc);
+    R al;
+    int n;
+    SweepR<R> lo;
+    const bool planned = fit_in && lower_planned && plan && plan->valid;
+    if (planned) {
+        lo.mb = (R)plan->low_mb;
+        lo.gravl = (R)plan->low_gravl;
+        lo.z = (R)plan->low_z;
+        lo.zend = (R)plan->low_zend;
+    } else {
+        al = rm::log(rm::fmin(alt, (R)105.0) / z1);
+        n = coarse_panels(al / step_lower);
+        if (n == 0) return kErrDomain;
+        lo = boole_sweep_r(z1, z1, rm::exp(al / (R)n), n, mb1 * grav_r(z1) / tloc1, true, tc);
+    }
     if (fit_in && lower_planned) {
         lo.sum = v7_series(JBT(kV7Sub2Lower), u);
         lo.tloc = v7_series(JBT(kV7Tloc2), u);
@@ -825,10 +884,16 @@ BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, do
         offset[5] = offset[4] - (R)25.0;
     } else {
         // 105 km -> min(alt, 500 km): the fixed six-panel plan at and above 500 km
-        al = rm::log(rm::fmin(alt, (R)500.0) / z);
-        n = coarse_panels(al / step_middle);
-        if (n == 0) return kErrDomain;
-        SweepR<R> mid = boole_sweep_r(z, lo.zend, rm::exp(al / (R)n), n, lo.gravl / tloc2, false, tc);
+        SweepR<R> mid;
+        if (planned && alt >= (R)500.0) {
+            mid.z = (R)plan->mid_z;
+            mid.zend = (R)plan->mid_zend;
+        } else {
+            al = rm::log(rm::fmin(alt, (R)500.0) / z);
+            n = coarse_panels(al / step_middle);
+            if (n == 0) return kErrDomain;
+            mid = boole_sweep_r(z, lo.zend, rm::exp(al / (R)n), n, lo.gravl / tloc2, false, tc);
+        }
         if (fit_in && lower_planned && alt >= (R)500.0) {
             mid.sum = v7_series(JBT(kV7Sub2Middle), u);
             mid.ain = v7_series(JBT(kV7AinMiddle), u);
@@ -866,35 +931,21 @@ BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, do
     // seasonal-latitudinal term, cut at 800 km by model 7
     R dlrsl = (R)0.0;
     if (!(v7 && alt >= (R)800.0)) {
-        const double years = (mjd - 36204.0) / 365.2422;
-        double capphi = years - ::trunc(years);
-        if (capphi == 0.0) capphi = ::copysign(0.0, years);
         const R sgn = lat_in >= 0.0 ? (R)1.0 : (R)-1.0;
         const R hm90 = alt - (R)90.0;
-        dlrsl = (R)0.02 * hm90 * rm::exp((R)-0.045 * hm90) * sgn * rm::sin((R)(kTwoPi * capphi + 1.72)) * slat *
-                slat;
+        dlrsl = (R)0.02 * hm90 * rm::exp((R)-0.045 * hm90) * sgn * E.sinphi * slat * slat;
     }
     // semiannual term (jb2008.rs:3436-3461)
     R dlrsa = (R)0.0;
     if (z < (R)2000.0) {
-        bool ok = true;
-        const double day = day_of_year(mjd, &ok);
-        if (!ok) return kErrDomain;
-        R fzm[5], gtm[10];
+        if (isnan(E.gtz)) return kErrDomain;  // the day is out of range
+        R fzm[5];
 #pragma unroll
         for (int i = 0; i < 5; ++i) fzm[i] = (R)JBT(kFzm)[i];
-#pragma unroll
-        for (int i = 0; i < 10; ++i) gtm[i] = (R)JBT(kGtm)[i];
         const R htz = alt / (R)1000.0;
         const R fz = f10b - (R)0.70 * s10b - (R)0.04 * m10b;
         const R fzz = fzm[0] + fz * (fzm[1] + htz * (fzm[2] + fzm[3] * htz + fzm[4] * fz));
-        const R fg = f10b - (R)0.75 * s10b - (R)0.37 * m10b;
-        R s1, c1;
-        rm::sincos((R)(kTwoPi * (day - 1.0) / 365.0), &s1, &c1);
-        const R s2 = (R)2.0 * s1 * c1, c2 = c1 * c1 - s1 * s1;
-        const R gtz = gtm[0] + gtm[1] * s1 + gtm[2] * c1 + gtm[3] * s2 + gtm[4] * c2 +
-                      fg * (gtm[5] + gtm[6] * s1 + gtm[7] * c1 + gtm[8] * s2 + gtm[9] * c2);
-        dlrsa = rm::fmax(fzz, (R)1.0e-6) * gtz;
+        dlrsa = rm::fmax(fzz, (R)1.0e-6) * E.gtz;
     }
     const R dlr = (R)kLn10 * (dlrsl + dlrsa);
     // compensated species sum
@@ -928,6 +979,48 @@ BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, do
     const double out = (double)(rho * fex);
     if (!(isfinite(out) && out > 0.0)) return kErrDomain;
     return out;
+}
+
+template <class R>
+BQP_HD double density_coarse_r(double mjd, double sun_dec, double hour_angle, double lat_in, double alt_m,
+                               const Drivers& din, int model) {
+    if (!isfinite(mjd) || !isfinite(sun_dec) || !isfinite(hour_angle) || !isfinite(lat_in) ||
+        !isfinite(alt_m) || !isfinite(din.f10) || !isfinite(din.f10b) || !isfinite(din.s10) ||
+        !isfinite(din.s10b) || !isfinite(din.m10) || !isfinite(din.m10b) || !isfinite(din.y10) ||
+        !isfinite(din.y10b) || !isfinite(din.dtc))
+        return kErrNonFinite;
+    if (alt_m < 90000.0) return kErrAltitude;
+    if (!(sun_dec >= -kPi / 2 && sun_dec <= kPi / 2) || !(lat_in >= -kPi / 2 && lat_in <= kPi / 2))
+        return kErrAngle;
+    if (din.f10 <= 0.0 || din.f10b <= 0.0 || din.s10 <= 0.0 || din.s10b <= 0.0 || din.m10 <= 0.0 ||
+        din.m10b <= 0.0 || din.y10 <= 0.0 || din.y10b <= 0.0)
+        return kErrIndex;
+    return density_coarse_core<R>(epoch_terms<R>(mjd, din, true), sun_dec, hour_angle, lat_in, alt_m, din, model,
+                                  nullptr);
+}
+
+// The plans' ends in R's arithmetic: the walks density_coarse_core makes at
+// 500 km (the nodes and what is kept of them do not depend on the profile tc).
+template <class R>
+inline CoarsePlan coarse_plan(int model) {
+    CoarsePlan P{};
+    if (model != 7) return P;
+    const R tc[4] = {(R)380.0, (R)10.7, (R)400.0, (R)0.027};
+    const R z1 = (R)90.0;
+    R al = rm::log((R)105.0 / z1);
+    int n = coarse_panels(al / (R)0.040);
+    const SweepR<R> lo = boole_sweep_r(z1, z1, rm::exp(al / (R)n), n, (R)0.0, true, tc);
+    al = rm::log((R)500.0 / lo.z);
+    n = coarse_panels(al / (R)0.300);
+    const SweepR<R> mid = boole_sweep_r(lo.z, lo.zend, rm::exp(al / (R)n), n, (R)0.0, false, tc);
+    P.low_z = lo.z;
+    P.low_zend = lo.zend;
+    P.low_mb = lo.mb;
+    P.low_gravl = lo.gravl;
+    P.mid_z = mid.z;
+    P.mid_zend = mid.zend;
+    P.valid = 1;
+    return P;
 }
 
 BQP_HD double density_coarse(double mjd, double sun_dec, double hour_angle, double lat, double alt_m,
@@ -1149,28 +1242,12 @@ __device__ __forceinline__ void cheb_eval_pair(double t, double* low, double* mi
 
 // fixed_fit: use the fixed-node sweep fits (c_fixed_fit) where they apply.
 template <int L>
-__device__ double density_group(double mjd, double sun_dec, double hour_angle, double lat, double alt_m,
+__device__ double density_group(const EpochR<double>& E, double sun_dec, double hour_angle, double lat, double alt_m,
                                 const Drivers& d, int q, unsigned gmask, bool fixed_fit,
                                 const JbFit2* fit2 = nullptr) {
     const JbFit* fit = fixed_fit ? &c_fixed_fit : nullptr;
-    double code = 0.0;
-    if (!isfinite(mjd) || !isfinite(sun_dec) || !isfinite(hour_angle) || !isfinite(lat) || !isfinite(alt_m) ||
-        !isfinite(d.f10) || !isfinite(d.f10b) || !isfinite(d.s10) || !isfinite(d.s10b) || !isfinite(d.m10) ||
-        !isfinite(d.m10b) || !isfinite(d.y10) || !isfinite(d.y10b) || !isfinite(d.dtc))
-        code = kErrNonFinite;
-    else if (alt_m < 90000.0)
-        code = kErrAltitude;
-    else if (!(sun_dec >= -kPi / 2 && sun_dec <= kPi / 2) || !(lat >= -kPi / 2 && lat <= kPi / 2))
-        code = kErrAngle;
-    else if (d.f10 <= 0.0 || d.f10b <= 0.0 || d.s10 <= 0.0 || d.s10b <= 0.0 || d.m10 <= 0.0 || d.m10b <= 0.0 ||
-             d.y10 <= 0.0 || d.y10b <= 0.0)
-        code = kErrIndex;
-    if (code != 0.0) return code;  // the whole group returns together
+    if (!geometry_valid(sun_dec, hour_angle, lat, alt_m)) return kErrDomain;  // the whole group returns together
     const double alt = alt_m / 1000.0;
-    const double fn = fmin(pow(d.f10b / 240.0, 0.25), 1.0);
-    const double fsb = d.f10b * fn + d.s10b * (1.0 - fn);
-    const double tsubc = 392.4 + 3.227 * fsb + 0.298 * (d.f10 - d.f10b) + 2.259 * (d.s10 - d.s10b) +
-                         0.312 * (d.m10 - d.m10b) + 0.178 * (d.y10 - d.y10b);
     const double eta = 0.5 * fabs(lat - sun_dec);
     const double theta = 0.5 * fabs(lat + sun_dec);
     double h = hour_angle;
@@ -1192,7 +1269,7 @@ __device__ double density_group(double mjd, double sun_dec, double hour_angle, d
     const double sin_theta = five_halves(sin(theta));
     const double cos_tau = fabs(cos(0.5 * tau));
     const double df = sin_theta + (cos_eta - sin_theta) * cos_tau * cos_tau * cos_tau;
-    const double tsubl = tsubc * (1.0 + 0.31 * df);
+    const double tsubl = E.tsubc * (1.0 + 0.31 * df);
     const double tinf = tsubl + d.dtc + dtc_correction(d.f10, st_hour, clat, alt);
     const double tsubx = 444.3807 + 0.02385 * tinf - 392.8292 * exp(-0.0021357 * tinf);
     const double gsubx = 0.054285714 * (tsubx - 183.0);
@@ -1232,11 +1309,12 @@ __device__ double density_group(double mjd, double sun_dec, double hour_angle, d
     double fact2 = anm / 28.960;
     const double fac[5] = {JBT(kFrac)[0] * fact2, fact2 * (1.0 + JBT(kFrac)[1]) - an, 2.0 * (an - fact2),
                            JBT(kFrac)[2] * fact2, JBT(kFrac)[3] * fact2};
-    double aln[6];
-    for (int i = 0; i < 5; ++i) aln[i] = fac[i] < 0.0 ? NAN : log(fac[i]);
+    // a species' number density is fac exp(off) (density() carries ln fac
+    // instead: five logarithms more, the same to the last bits of ln fac)
+    double off[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     double z = lo.z;
     if (alt <= 105.0) {
-        aln[5] = aln[4] - 25.0;
+        off[5] = -25.0;
     } else {
         SweepG mid;
         if (use_fit && alt >= 500.0) {
@@ -1283,39 +1361,32 @@ __device__ double density_group(double mjd, double sun_dec, double hour_angle, d
             fact2 = (mid.sum + up.sum) / kRstar;
             hsign = -1.0;
         }
-        for (int i = 0; i < 4; ++i) aln[i] = aln[i] - altr - fact2 * JBT(kAmw)[i];
-        aln[4] = aln[4] - (1.0 - 0.38) * altr - fact2 * JBT(kAmw)[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) off[i] = -altr - fact2 * JBT(kAmw)[i];
+        off[4] = -(1.0 - 0.38) * altr - fact2 * JBT(kAmw)[4];
         const double al10t5 = log10(tinf);
         const double alnh5 = (5.5 * al10t5 - 39.40) * al10t5 + 73.13;
-        aln[5] = kLn10 * (alnh5 + 6.0) + hsign * (log(tloc4 / tloc3) + up.sum * JBT(kAmw)[5] / kRstar);
+        off[5] = kLn10 * (alnh5 + 6.0) + hsign * (log(tloc4 / tloc3) + up.sum * JBT(kAmw)[5] / kRstar);
     }
-    const double years = (mjd - 36204.0) / 365.2422;
-    double capphi = years - trunc(years);
-    if (capphi == 0.0) capphi = copysign(0.0, years);
     const double sgn = lat >= 0.0 ? 1.0 : -1.0;
     const double hm90 = alt - 90.0;
-    const double dlrsl = 0.02 * hm90 * exp(-0.045 * hm90) * sgn * sin(kTwoPi * capphi + 1.72) * slat * slat;
+    const double dlrsl = 0.02 * hm90 * exp(-0.045 * hm90) * sgn * E.sinphi * slat * slat;
     double dlrsa = 0.0;
     if (z < 2000.0) {
-        bool ok = true;
-        const double day = day_of_year(mjd, &ok);
-        if (!ok) return kErrDomain;
+        if (isnan(E.gtz)) return kErrDomain;  // the day is out of range
         const double htz = alt / 1000.0;
-        double fsmb = d.f10b - 0.70 * d.s10b - 0.04 * d.m10b;
+        const double fsmb = d.f10b - 0.70 * d.s10b - 0.04 * d.m10b;
         const double fzz = JBT(kFzm)[0] + JBT(kFzm)[1] * fsmb + JBT(kFzm)[2] * fsmb * htz +
                            JBT(kFzm)[3] * fsmb * htz * htz + JBT(kFzm)[4] * fsmb * fsmb * htz;
-        fsmb = d.f10b - 0.75 * d.s10b - 0.37 * d.m10b;
-        double s1, c1;
-        sincos(kTwoPi * (day - 1.0) / 365.0, &s1, &c1);
-        const double s2 = 2.0 * s1 * c1, c2 = c1 * c1 - s1 * s1;
-        const double gtz = JBT(kGtm)[0] + JBT(kGtm)[1] * s1 + JBT(kGtm)[2] * c1 + JBT(kGtm)[3] * s2 +
-                           JBT(kGtm)[4] * c2 + JBT(kGtm)[5] * fsmb + JBT(kGtm)[6] * fsmb * s1 +
-                           JBT(kGtm)[7] * fsmb * c1 + JBT(kGtm)[8] * fsmb * s2 + JBT(kGtm)[9] * fsmb * c2;
-        dlrsa = fmax(fzz, 1.0e-6) * gtz;
+        dlrsa = fmax(fzz, 1.0e-6) * E.gtz;
     }
     const double dlr = kLn10 * (dlrsl + dlrsa);
     double sumnm = 0.0;
-    for (int i = 0; i < 6; ++i) sumnm += exp(aln[i] + dlr) * JBT(kAmw)[i];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const double f = i < 5 ? fac[i] : (alt <= 105.0 ? fac[4] : 1.0);
+        sumnm += (f < 0.0 ? NAN : f) * exp(off[i] + dlr) * JBT(kAmw)[i];
+    }
     rho = sumnm / kAvogadro;
     double fex = 1.0;
     if (alt >= 1000.0 && alt < 1500.0) {

@@ -59,6 +59,7 @@ struct ForceParams {
     EphemTable eph_sun, eph_moon;  // precomputed catalogues (n 0: the analytic series)
     const jb::JbFit* fit;  // device copy of the fixed-node sweep fits, or null
     const jb::JbFit2* fit2;  // altitude-dependent sweep fits (stage-synchronous drag), or null
+    jb::CoarsePlan plan;     // the ends of model 7's fixed plans
     ft::FrameTab frame;      // IAU 2006/2000A segments (frame.mode 1) or the GMST rotation (0)
 };
 

@@ -93,8 +93,8 @@ struct KernelTimes {
     int64_t launches[kKcCount];
 };
 
-size_t pipeline_bytes(int64_t cap, int iau);
-void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau);
+size_t pipeline_bytes(int64_t cap, int iau, int drag);
+void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau, int drag);
 cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st,
                             double max_seconds, int gravity_threads, int gravity_slots,
                             KernelTimes* times = nullptr);

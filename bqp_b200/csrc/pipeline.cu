@@ -87,8 +87,13 @@ struct StageTimes {
     __device__ __forceinline__ double& jd(int slot) const { return at(12, slot); }
     // GMST: sin, cos; IAU: R (row-major) and the ITRS angular velocity (GCRS)
     __device__ __forceinline__ double& frame(int i, int slot) const { return at(13 + i, slot); }
+    // with drag, the last six: the Sun's Earth-fixed x and y, its declination,
+    // and jb::EpochR (tsubc NaN: no or invalid drivers)
+    __device__ __forceinline__ double& drag(const PipeBufs& P, int i, int slot) const {
+        return at(P.fields - 6 + i, slot);
+    }
 };
-constexpr int kTimesGmst = 15, kTimesIau = 25;
+constexpr int kTimesFields = 13, kTimesGmst = 2, kTimesIau = 12, kTimesDrag = 6;
 
 // Sum of the stage-`st` force terms into K(st, 3..5).
 __device__ __forceinline__ void finish_stage(const PipeBufs& P, int st, int slot) {
@@ -194,6 +199,35 @@ __global__ void __launch_bounds__(kBlock) pl_times(PropArgs A, PipeBufs P, int c
         double sun[3];
         sun_at(fp.eph_sun, jd, sun);
         for (int i = 0; i < 3; ++i) Q.sun(i, slot) = sun[i];
+        if (fp.drag) {
+            // JB2008 adapter (rhs.rs:3551-3776), as Encke::density_at: the
+            // Sun's side of it and the drivers'
+            double si[3];
+            slot_to_itrs(P, Q, slot, sun, si);
+            const double sun_r = sqrt(fma(si[0], si[0], fma(si[1], si[1], si[2] * si[2])));
+            Q.drag(P, 0, slot) = si[0];
+            Q.drag(P, 1, slot) = si[1];
+            Q.drag(P, 2, slot) = asin(fmin(1.0, fmax(-1.0, si[2] / sun_r)));
+            jb::Drivers dr = fp.drivers;
+            const double mjd = jd - 2400000.5;
+            double tsubc = NAN, sinphi = 0.0, gtz = 0.0;
+            if ((fp.dtab.n_solar == 0 || jb::lookup_drivers(fp.dtab, jd, &dr)) && jb::drivers_valid(mjd, dr)) {
+                if (fp.drag_fp32) {
+                    const jb::EpochR<float> E = jb::epoch_terms<float>(mjd, dr, true);
+                    tsubc = E.tsubc;
+                    sinphi = E.sinphi;
+                    gtz = E.gtz;
+                } else {
+                    const jb::EpochR<double> E = jb::epoch_terms<double>(mjd, dr, fp.atm_model != 4);
+                    tsubc = E.tsubc;
+                    sinphi = E.sinphi;
+                    gtz = E.gtz;
+                }
+            }
+            Q.drag(P, 3, slot) = tsubc;
+            Q.drag(P, 4, slot) = sinphi;
+            Q.drag(P, 5, slot) = gtz;
+        }
     }
     if (fp.moon) {
         double moon[3];
@@ -397,7 +431,8 @@ __global__ void __launch_bounds__(kBlock) pl_sur_check(PipeBufs P, int cur, doub
 // [0, nb_hi) take list 0 with LH lanes per state, the rest list 1 with LL),
 // so that a stage's states are resident together in as few waves as the
 // register budget allows.
-template <int L, bool kCoarse = false>
+// kForm 0: the exact model; 1, 2: the coarse profiles in FP64 and in FP32.
+template <int L, int kForm = 0>
 __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs& P, int st, int list, int block) {
     const int gt = block * blockDim.x + threadIdx.x;
     const int item = gt / L;
@@ -412,34 +447,34 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
     if (cd != 0.0 && am != 0.0) {
         // JB2008 adapter (rhs.rs:3551-3776), as Encke::density_at
         const StageTimes Q(P, st);
-        const double sun[3] = {Q.sun(0, slot), Q.sun(1, slot), Q.sun(2, slot)};
-        const double jd = Q.jd(slot);
-        double pi[3], si[3];
+        double pi[3];
         slot_to_itrs(P, Q, slot, sp, pi);
-        slot_to_itrs(P, Q, slot, sun, si);
-        const double sun_r = sqrt(fma(si[0], si[0], fma(si[1], si[1], si[2] * si[2])));
         const double sat_r = sqrt(fma(pi[0], pi[0], fma(pi[1], pi[1], pi[2] * pi[2])));
         double rho;
         if ((sat_r - fp.earth_radius) * 1000.0 > 2500.0e3) {
             rho = 1.0e-19;
         } else {
+            const double si0 = Q.drag(P, 0, slot), si1 = Q.drag(P, 1, slot), dec = Q.drag(P, 2, slot);
+            const jb::EpochR<double> E{Q.drag(P, 3, slot), Q.drag(P, 4, slot), Q.drag(P, 5, slot)};
             const double alt_m = geodetic_altitude_km(pi[0], pi[1], pi[2], fp.earth_radius) * 1000.0;
-            const double dec = asin(fmin(1.0, fmax(-1.0, si[2] / sun_r)));
-            const double ha = atan2(fma(pi[1], si[0], -(pi[0] * si[1])), fma(pi[0], si[0], pi[1] * si[1]));
+            const double ha = atan2(fma(pi[1], si0, -(pi[0] * si1)), fma(pi[0], si0, pi[1] * si1));
             const double lat = asin(fmin(1.0, fmax(-1.0, pi[2] / sat_r)));
             jb::Drivers dr = fp.drivers;
+            if (fp.dtab.n_solar > 0) jb::lookup_drivers(fp.dtab, Q.jd(slot), &dr);
             // fixed-node fits from constant memory (fp.fit holds the same numbers);
             // no drivers at this instant -> NaN density (rhs.rs:3560-3571), the
             // same verdict on every lane of the group
-            if (fp.dtab.n_solar > 0 && !jb::lookup_drivers(fp.dtab, jd, &dr))
+            if (isnan(E.tsubc))
                 rho = NAN;
-            else if (kCoarse && fp.drag_fp32)
-                rho = jb::density_coarse_r<float>(jd - 2400000.5, dec, ha, lat, alt_m, dr, fp.atm_model);
-            else if (kCoarse)
-                rho = jb::density_coarse(jd - 2400000.5, dec, ha, lat, alt_m, dr, fp.atm_model);
+            else if (kForm == 0)
+                rho = jb::density_group<L>(E, dec, ha, lat, alt_m, dr, q, gmask, fp.fit != nullptr, fp.fit2);
+            else if (!jb::geometry_valid(dec, ha, lat, alt_m))
+                rho = NAN;
+            else if (kForm == 2)
+                rho = jb::density_coarse_core<float>({(float)E.tsubc, (float)E.sinphi, (float)E.gtz}, dec, ha, lat,
+                                                     alt_m, dr, fp.atm_model, &fp.plan);
             else
-                rho = jb::density_group<L>(jd - 2400000.5, dec, ha, lat, alt_m, dr, q, gmask,
-                                           fp.fit != nullptr, fp.fit2);
+                rho = jb::density_coarse_core<double>(E, dec, ha, lat, alt_m, dr, fp.atm_model, &fp.plan);
             if (!(rho > 0.0) || !isfinite(rho)) rho = NAN;
             else if (alt_m > 2500.0e3) rho = fmin(rho, 1.0e-19);
         }
@@ -482,9 +517,10 @@ __global__ void __launch_bounds__(kBlock, BQP_DRAG_MIN_BLOCKS) pl_drag(ForcePara
 
 // The coarse profiles (atm_model 5-7): a short chain per state, one lane
 // each, both altitude lists in one launch.
+template <int kForm>
 __global__ void __launch_bounds__(kBlock) pl_drag_coarse(ForceParams fp, PipeBufs P, int st, int nb_hi) {
-    if ((int)blockIdx.x < nb_hi) drag_rows<1, true>(fp, P, st, 0, blockIdx.x);
-    else drag_rows<1, true>(fp, P, st, 1, blockIdx.x - nb_hi);
+    if ((int)blockIdx.x < nb_hi) drag_rows<1, kForm>(fp, P, st, 0, blockIdx.x);
+    else drag_rows<1, kForm>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
 // ------------------------------------------------------------------ control
@@ -621,7 +657,7 @@ __global__ void __launch_bounds__(kBlock) pl_abort(PropArgs A, PipeBufs P, int c
 
 // ------------------------------------------------------------------- host
 // Stages whose instants are prepared at once: as many as leave their
-// quantities (200 B a row and stage, 120 in the GMST frame) in L2 beside what
+// quantities (248 B a row and stage, 168 in the GMST frame) in L2 beside what
 // the stages themselves touch, at least one.  The ring has one more, the
 // stage before a group, which is finished after the group is prepared.
 static int times_group(int64_t cap, int fields) {
@@ -630,13 +666,13 @@ static int times_group(int64_t cap, int fields) {
     return (int)(g < 1 ? 1 : (g > kStageBufs ? kStageBufs : g));
 }
 
-size_t pipeline_bytes(int64_t cap, int iau) {
+size_t pipeline_bytes(int64_t cap, int iau, int drag) {
     PipeBufs P{};
-    pipeline_carve(P, nullptr, cap, iau);
+    pipeline_carve(P, nullptr, cap, iau, drag);
     return (size_t)(uintptr_t)P.dcount + 2 * (size_t)P.ring * sizeof(int32_t) + 256;
 }
 
-void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau) {
+void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau, int drag) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
         off = (off + 255) & ~(size_t)255;
@@ -653,7 +689,7 @@ void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau) {
     P.k = (double*)take((size_t)kStageBufs * 6 * c * 8);
     P.sp = (double*)take(6 * c * 8);
     P.iau = iau;
-    P.fields = iau ? kTimesIau : kTimesGmst;
+    P.fields = kTimesFields + (iau ? kTimesIau : kTimesGmst) + (drag ? kTimesDrag : 0);
     P.ring = times_group(cap, P.fields) + 1;
     P.tq = (double*)take((size_t)P.ring * P.fields * c * 8);
     P.part = (double*)take(3 * c * 8);
@@ -779,8 +815,10 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
                     if (A.force.atm_model == 4)
                         pl_drag<kLanesHigh, kLanesLow>
                             <<<dblocks_hi + dblocks_lo, kBlock, 0, st>>>(A.force, P, s, dblocks_hi);
+                    else if (A.force.drag_fp32)
+                        pl_drag_coarse<2><<<2 * blocks, kBlock, 0, st>>>(A.force, P, s, blocks);
                     else
-                        pl_drag_coarse<<<2 * blocks, kBlock, 0, st>>>(A.force, P, s, blocks);
+                        pl_drag_coarse<1><<<2 * blocks, kBlock, 0, st>>>(A.force, P, s, blocks);
                 });
         }
         timed(kKcControl, [&] { pl_control<M><<<blocks, kBlock, 0, st>>>(A, P, cur, dense ? 1 : 0, timed_out); });
