@@ -41,11 +41,12 @@ constexpr int kBlock = 256;
 
 // Drag lanes per state above and below ~510 km (the lanes share the sweep
 // series and the intervals walked exactly), and the drag kernel's minimum
-// resident CTAs per SM, which sets its register budget (3: 80 registers, a
-// few hundred bytes spilled).  Measured on 65,536 LEO states at 70x70: one
-// lane above 510 km and four below, both lists in one launch at 3 CTAs per
-// SM, fit every state of a stage in one wave; that took the drag kernels
-// from 1,023 ms to 701 ms per 5,400 s segment.
+// resident CTAs per SM, which sets its register budget.  The stage's drag runs
+// beside its gravity, which leaves it half of an SM's registers (128 threads
+// of 248): 65,536 rows at 70x70, exact model, us a pass: 327,168 with 80
+// registers (6 CTAs of 128), 332,036 with 64, 333,552 with 96, 331,616 with
+// 128; one after the other 398,180.  Where all rows fit in a wave anyway, 128
+// registers and no spills: 7,000 rows 188,420 us against 207,638.
 #ifndef BQP_DRAG_LANES_HIGH
 #define BQP_DRAG_LANES_HIGH 1
 #endif
@@ -53,8 +54,15 @@ constexpr int kBlock = 256;
 #define BQP_DRAG_LANES_LOW 4
 #endif
 #ifndef BQP_DRAG_MIN_BLOCKS
-#define BQP_DRAG_MIN_BLOCKS 3
+#define BQP_DRAG_MIN_BLOCKS 6
 #endif
+#ifndef BQP_DRAG_MIN_BLOCKS_FEW
+#define BQP_DRAG_MIN_BLOCKS_FEW 4
+#endif
+#ifndef BQP_DRAG_BLOCK
+#define BQP_DRAG_BLOCK 128
+#endif
+constexpr int kDragBlock = BQP_DRAG_BLOCK;
 // stage derivative buffers per row: the most stages of any tableau (Vern9's
 // 16) plus the dense-output stage of the sampled non-FSAL path
 constexpr int kStageBufs = Tab<kVern9>::S + 1;
@@ -509,16 +517,19 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
         for (int i = 0; i < 3; ++i) P.adrag[(size_t)i * P.cap + slot] = a[i];
 }
 
-template <int LH, int LL>
-__global__ void __launch_bounds__(kBlock, BQP_DRAG_MIN_BLOCKS) pl_drag(ForceParams fp, PipeBufs P, int st, int nb_hi) {
+template <int LH, int LL, int kMinBlocks>
+__global__ void __launch_bounds__(kDragBlock, kMinBlocks) pl_drag(ForceParams fp, PipeBufs P, int st, int nb_hi) {
     if ((int)blockIdx.x < nb_hi) drag_rows<LH>(fp, P, st, 0, blockIdx.x);
     else drag_rows<LL>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
 // The coarse profiles (atm_model 5-7): a short chain per state, one lane
 // each, both altitude lists in one launch.
+#ifndef BQP_COARSE_MIN_BLOCKS
+#define BQP_COARSE_MIN_BLOCKS 4
+#endif
 template <int kForm>
-__global__ void __launch_bounds__(kBlock) pl_drag_coarse(ForceParams fp, PipeBufs P, int st, int nb_hi) {
+__global__ void __launch_bounds__(kDragBlock, BQP_COARSE_MIN_BLOCKS) pl_drag_coarse(ForceParams fp, PipeBufs P, int st, int nb_hi) {
     if ((int)blockIdx.x < nb_hi) drag_rows<1, kForm>(fp, P, st, 0, blockIdx.x);
     else drag_rows<1, kForm>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
@@ -720,13 +731,22 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     const int groups = (stages + P.ring - 2) / (P.ring - 1), group = (stages + groups - 1) / groups;
     const int blocks = (int)((A.n + kBlock - 1) / kBlock);
     constexpr int kLanesHigh = BQP_DRAG_LANES_HIGH, kLanesLow = BQP_DRAG_LANES_LOW;
-    const int dblocks_hi = (int)((A.n * kLanesHigh + kBlock - 1) / kBlock);
-    const int dblocks_lo = (int)((A.n * kLanesLow + kBlock - 1) / kBlock);
+    const int dblocks_hi = (int)((A.n * kLanesHigh + kDragBlock - 1) / kDragBlock);
+    const int dblocks_lo = (int)((A.n * kLanesLow + kDragBlock - 1) / kDragBlock);
+    // more registers a thread while a stage's rows still fit in one wave
+    auto dker = dblocks_hi <= 2 * device_sm_count() ? pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS_FEW>
+                                                    : pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS>;
+    const int cblocks = (int)((A.n + kDragBlock - 1) / kDragBlock);
     // with the surrogate, the exact stage covers only the degrees it leaves out
     const bool sur = A.sur.P != nullptr;
     const GravTable GT = sur ? A.sur.low : A.grav;
     // the surrogate's residual check also runs the whole exact field
     const bool check = sur && A.sur.check > 0.0;
+    // with drag beside it, 128 threads (31 K registers an SM) leave the other
+    // half of the registers to the drag kernel, and four warps of four rows a
+    // lane still keep the FP64 pipe as busy as the table reads let it: 65,536
+    // rows 331 ms a pass against 398 with 256 threads, 20,001 rows 179 and 210
+    if (A.force.drag && !times && gthreads == 256) gthreads = 128;
     GravLaunch G = gravity_launch(GT, A.n, device_sm_count(), gthreads, gslots);
     GravLaunch GF = check ? gravity_launch(A.sur.full, A.n, device_sm_count(), gthreads, gslots) : G;
     auto gker = pl_gravity_of(G), gker_full = pl_gravity_of(GF);
@@ -748,10 +768,22 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
 
     // private stream ordered after the caller's stream (graphs need a
     // capturable stream)
-    cudaStream_t st;
-    e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    // and a second one, whose kernels give way to the first's: a stage's drag
+    // runs beside its gravity (one after the other while kernels are timed)
+    int prio_low = 0, prio_high = 0;
+    cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
+    cudaStream_t st, st2;
+    e = cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, prio_high);
     if (e != cudaSuccess) return e;
-    cudaEvent_t ev_in, ev_out, ev_cnt;
+    e = cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, prio_low);
+    if (e != cudaSuccess) {
+        cudaStreamDestroy(st);
+        return e;
+    }
+    const bool beside = A.force.drag && A.force.gravity_on && !times;
+    cudaEvent_t ev_in, ev_out, ev_cnt, ev_fork, ev_join;
+    cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming);
     cudaEventCreateWithFlags(&ev_cnt, cudaEventDisableTiming);
@@ -791,6 +823,12 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
                     pl_times<M><<<dim3(blocks, std::min(group, stages - s)), kBlock, 0, st>>>(A, P, cur, s);
                 pl_prep<M><<<blocks, kBlock, 0, st>>>(A, P, cur, s);
             });
+            cudaStream_t sd = st;
+            if (beside) {
+                sd = st2;
+                cudaEventRecord(ev_fork, st);
+                cudaStreamWaitEvent(st2, ev_fork, 0);
+            }
             if (A.force.gravity_on)
                 timed(kKcGravity, [&] {
                     gravity_run(G, gker, gctas, st, GT, G.aux, P, cur, s, P.agrav, nullptr, nullptr);
@@ -813,13 +851,16 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
             if (A.force.drag)
                 timed(kKcDrag, [&] {
                     if (A.force.atm_model == 4)
-                        pl_drag<kLanesHigh, kLanesLow>
-                            <<<dblocks_hi + dblocks_lo, kBlock, 0, st>>>(A.force, P, s, dblocks_hi);
+                        dker<<<dblocks_hi + dblocks_lo, kDragBlock, 0, sd>>>(A.force, P, s, dblocks_hi);
                     else if (A.force.drag_fp32)
-                        pl_drag_coarse<2><<<2 * blocks, kBlock, 0, st>>>(A.force, P, s, blocks);
+                        pl_drag_coarse<2><<<2 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
                     else
-                        pl_drag_coarse<1><<<2 * blocks, kBlock, 0, st>>>(A.force, P, s, blocks);
+                        pl_drag_coarse<1><<<2 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
                 });
+            if (beside) {
+                cudaEventRecord(ev_join, st2);
+                cudaStreamWaitEvent(st, ev_join, 0);
+            }
         }
         timed(kKcControl, [&] { pl_control<M><<<blocks, kBlock, 0, st>>>(A, P, cur, dense ? 1 : 0, timed_out); });
     };
@@ -884,6 +925,9 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     cudaEventDestroy(ev_in);
     cudaEventDestroy(ev_out);
     cudaEventDestroy(ev_cnt);
+    cudaEventDestroy(ev_fork);
+    cudaEventDestroy(ev_join);
+    cudaStreamDestroy(st2);
     cudaStreamDestroy(st);
     return e;
 }
