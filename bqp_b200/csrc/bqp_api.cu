@@ -532,6 +532,7 @@ struct bqp_ctx {
     Coeffs coeffs;
     int parsed_order = 0;
     double* d_tab = nullptr;
+    double* d_tab_cells = nullptr;  // the same field as cells (sigma points in the GMST frame)
     int ncells = 0;
     size_t tab_bytes = 0;
     int use_smem = 0;
@@ -838,6 +839,8 @@ int upload_table(bqp_ctx* ctx) {
     ctx->use_smem = ctx->tab_bytes <= kSmemLimit ? 1 : 0;
     if (ctx->d_tab) cudaFree(ctx->d_tab);
     ctx->d_tab = nullptr;
+    if (ctx->d_tab_cells) cudaFree(ctx->d_tab_cells);
+    ctx->d_tab_cells = nullptr;
     cudaError_t e = cudaMalloc(&ctx->d_tab, ctx->tab_bytes);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(gravity table)");
     e = cudaMemcpy(ctx->d_tab, tab.data(), ctx->tab_bytes, cudaMemcpyHostToDevice);
@@ -874,6 +877,25 @@ int upload_table(bqp_ctx* ctx) {
         ctx->split_ls = ls;
         ctx->split_bytes = (uint32_t)buf.size();
     }
+    return 0;
+}
+
+// The FP64 field as a table of cells (PropArgs::ordered), built at its first
+// use and dropped with the field's other tables.
+int cells_table(bqp_ctx* ctx, GravTable& T) {
+    const int N = ctx->cfg.order;
+    const size_t bytes = (size_t)gravity_cells(N) * kCellDoubles * sizeof(double);
+    if (!ctx->d_tab_cells) {
+        const std::vector<long double> v = gravity_cell_values(ctx->coeffs, N);
+        const std::vector<double> tab(v.begin(), v.end());
+        cudaError_t e = cudaMalloc(&ctx->d_tab_cells, bytes);
+        if (e == cudaSuccess) e = cudaMemcpy(ctx->d_tab_cells, tab.data(), bytes, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(e, "gravity cells");
+    }
+    T.tab = ctx->d_tab_cells;
+    T.bytes = (uint32_t)bytes;
+    T.in_smem = bytes <= kSmemLimit ? 1 : 0;
+    T.cells = 1;
     return 0;
 }
 
@@ -931,7 +953,7 @@ int set_device(const bqp_ctx* ctx) {
 
 int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, const double* epoch,
                 double t0, const double* tf, const double* ballistic, int32_t n_t, const double* t_eval,
-                int32_t out_mode, double* out, int32_t* status, int64_t* steps, int64_t* evals) {
+                int32_t out_mode, double* out, int32_t* status, int64_t* steps, int64_t* evals, bool sigma = false) {
     PropArgs A{};
     A.n = n;
     A.in = in;
@@ -959,6 +981,11 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
     A.fit_host = A.force.fit ? &ctx->h_fit : nullptr;
     A.ctrl = ctrl_params(ctx);
     A.grav = grav_table(ctx);
+    if (sigma && A.force.frame.mode == 0 && A.grav.ls == 0 && !ctx->cfg.surrogate) {
+        A.ordered = 1;
+        A.force.plan.valid = 0;
+        if (int rc = cells_table(ctx, A.grav)) return rc;
+    }
     if (ctx->cfg.surrogate) {
         if (int rc = surrogate_stage_args(ctx, A.sur)) return rc;
     }
@@ -1265,6 +1292,7 @@ int bqp_ctx_destroy(bqp_ctx* ctx) {
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     else cudaDeviceSynchronize();
     if (ctx->d_tab) cudaFree(ctx->d_tab);
+    if (ctx->d_tab_cells) cudaFree(ctx->d_tab_cells);
     if (ctx->d_queue) cudaFree(ctx->d_queue);
     if (ctx->d_ecl) cudaFree(ctx->d_ecl);
     if (ctx->d_ws) cudaFree(ctx->d_ws);
@@ -2014,7 +2042,7 @@ int sigma_run(bqp_ctx* ctx, int64_t n, const SigmaSet& SS, int32_t set, const Si
                              B.rows, B.row_epoch, B.row_tf, bal ? B.row_bal : nullptr, status, s);
     if (e != cudaSuccess) return cuda_fail(e, "sigma-point generation");
     int rc = launch_prop(ctx, n * SS.points, B.rows, 0, B.row_epoch, t0, B.row_tf, bal ? B.row_bal : nullptr, 0,
-                         nullptr, 0, B.out_rows, B.row_status, nullptr, B.row_evals);
+                         nullptr, 0, B.out_rows, B.row_status, nullptr, B.row_evals, true);
     if (rc) return rc;
     e = launch_sigma_recombine(n, SS.points, B.wm, B.wc, B.out_rows, B.row_status, B.row_evals, mean_out, cov_out,
                                status, evals, s);

@@ -298,6 +298,131 @@ BQP_HD int gravity_part_column(int order, int p, int parts) {
 }
 
 // ---------------------------------------------------------------------------
+// The FP64 field with V and W both carried down every column and both
+// multiplied by their weights in every cell (12 operations a cell), over the
+// columns [j0, j1) of a table of cells {a, b, Ax, Bx, Ay, By, Az, Bz}.  Only
+// sigma-point rows in the GMST frame take it (PropArgs::ordered), for the
+// order in which it adds.
+template <int NT>
+BQP_HD void gravity_columns(const double* __restrict__ tab, int order, int j0, int j1, const double* px,
+                            const double* py, const double* pz, double (*acc)[3]) {
+    double xc[NT], yc[NT], zc[NT], c2re[NT], vd[NT], wd[NT], ax[NT], ay[NT], az[NT];
+#pragma unroll
+    for (int q = 0; q < NT; ++q) {
+        const double r2 = fma(px[q], px[q], fma(py[q], py[q], pz[q] * pz[q]));
+        const double c2 = kReGravity / r2;
+        xc[q] = px[q] * c2;
+        yc[q] = py[q] * c2;
+        zc[q] = pz[q] * c2;
+        c2re[q] = c2 * kReGravity;
+        vd[q] = sqrt(c2re[q]);
+        wd[q] = 0.0;
+        ax[q] = ay[q] = az[q] = 0.0;
+    }
+    const int last = order + 1;
+    const double2* tab2 = reinterpret_cast<const double2*>(tab);
+    for (int j = 1; j < j0; ++j) {
+        const double a = tab2[(size_t)gravity_col_offset(order, j) * 4].x;
+#pragma unroll
+        for (int q = 0; q < NT; ++q) {
+            const double nv = a * fma(xc[q], vd[q], -yc[q] * wd[q]);
+            const double nw = a * fma(xc[q], wd[q], yc[q] * vd[q]);
+            vd[q] = nv;
+            wd[q] = nw;
+        }
+    }
+    const double2* cell = tab2 + (size_t)gravity_col_offset(order, j0) * 4;
+    for (int j = j0; j < j1; ++j) {
+        {
+            const double2 ab = cell[0], wx = cell[1], wy = cell[2], wz = cell[3];
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                if (j > 0) {
+                    const double nv = ab.x * fma(xc[q], vd[q], -yc[q] * wd[q]);
+                    const double nw = ab.x * fma(xc[q], wd[q], yc[q] * vd[q]);
+                    vd[q] = nv;
+                    wd[q] = nw;
+                }
+                ax[q] = fma(wx.x, vd[q], fma(wx.y, wd[q], ax[q]));
+                ay[q] = fma(wy.x, vd[q], fma(wy.y, wd[q], ay[q]));
+                az[q] = fma(wz.x, vd[q], fma(wz.y, wd[q], az[q]));
+            }
+            cell += 4;
+        }
+        if (j == last) break;
+        double v0[NT], w0[NT], v1[NT], w1[NT];
+        {
+            const double2 ab = cell[0], wx = cell[1], wy = cell[2], wz = cell[3];
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                const double a = ab.x * zc[q];
+                v0[q] = vd[q];
+                w0[q] = wd[q];
+                v1[q] = a * vd[q];
+                w1[q] = a * wd[q];
+                ax[q] = fma(wx.x, v1[q], fma(wx.y, w1[q], ax[q]));
+                ay[q] = fma(wy.x, v1[q], fma(wy.y, w1[q], ay[q]));
+                az[q] = fma(wz.x, v1[q], fma(wz.y, w1[q], az[q]));
+            }
+            cell += 4;
+        }
+        // interior rows j+2..last, two per iteration (the row registers
+        // rotate without moves); the next pair is in flight meanwhile
+        const int pairs = (last - j - 1) >> 1;
+        double2 nx[8];
+        if (pairs > 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) nx[i] = cell[i];
+        }
+#pragma unroll 2
+        for (int p = 0; p < pairs; ++p) {
+            double2 cb[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) cb[i] = nx[i];
+            if (p + 1 < pairs) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) nx[i] = cell[8 + i];
+            }
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                const double ta = cb[0].x * zc[q], tb = cb[0].y * c2re[q];
+                v0[q] = fma(ta, v1[q], -tb * v0[q]);
+                w0[q] = fma(ta, w1[q], -tb * w0[q]);
+                ax[q] = fma(cb[1].x, v0[q], fma(cb[1].y, w0[q], ax[q]));
+                ay[q] = fma(cb[2].x, v0[q], fma(cb[2].y, w0[q], ay[q]));
+                az[q] = fma(cb[3].x, v0[q], fma(cb[3].y, w0[q], az[q]));
+                const double ta2 = cb[4].x * zc[q], tb2 = cb[4].y * c2re[q];
+                v1[q] = fma(ta2, v0[q], -tb2 * v1[q]);
+                w1[q] = fma(ta2, w0[q], -tb2 * w1[q]);
+                ax[q] = fma(cb[5].x, v1[q], fma(cb[5].y, w1[q], ax[q]));
+                ay[q] = fma(cb[6].x, v1[q], fma(cb[6].y, w1[q], ay[q]));
+                az[q] = fma(cb[7].x, v1[q], fma(cb[7].y, w1[q], az[q]));
+            }
+            cell += 8;
+        }
+        if ((last - j - 1) & 1) {
+            const double2 ab = cell[0], wx = cell[1], wy = cell[2], wz = cell[3];
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                const double ta = ab.x * zc[q], tb = ab.y * c2re[q];
+                const double v2 = fma(ta, v1[q], -tb * v0[q]);
+                const double w2 = fma(ta, w1[q], -tb * w0[q]);
+                ax[q] = fma(wx.x, v2, fma(wx.y, w2, ax[q]));
+                ay[q] = fma(wy.x, v2, fma(wy.y, w2, ay[q]));
+                az[q] = fma(wz.x, v2, fma(wz.y, w2, az[q]));
+            }
+            cell += 4;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NT; ++q) {
+        acc[q][0] = ax[q];
+        acc[q][1] = ay[q];
+        acc[q][2] = az[q];
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Split-precision form.  Cell (l, j) carries only degree n = l - 1, so rows
 // l <= ls hold degrees n <= ls - 1 (the central-field corrections J2...,
 // kept in FP64) and every other cell the higher degrees, evaluated in FP32:

@@ -10,7 +10,8 @@
 // one of them over distributed shared memory.  See gravity_launch and
 // gravity_plan for how the split is picked.
 //
-// Split-precision field: the CTA is cut into `parts` groups of `tpart`
+// Split-precision field, and the FP64 field in the order of its cells
+// (GravTable::cells): the CTA is cut into `parts` groups of `tpart`
 // threads, every group evaluates all rows of a pass over its own run of
 // columns, and the partial sums are added in shared memory.
 #pragma once
@@ -130,7 +131,8 @@ struct GravTable {
     int order;
     int ls;          // 0: plain FP64; else the last FP64 row
     uint32_t bytes;  // size of tab (plain form: without its pad)
-    int in_smem;     // split form: 1 if staged into shared memory per CTA
+    int in_smem;     // split form and cells: 1 if staged into shared memory per CTA
+    int cells;       // 1: plain FP64 cells {a, b, Ax .. Bz} (gravity_columns), in every column
 };
 
 inline uint32_t gravity_table_bytes(int order, int ls) {
@@ -454,7 +456,11 @@ __device__ __forceinline__ void gravity_cta_split(const GravTable& T, int parts_
         }
         if (member) {
             const size_t lo_doubles = (size_t)split_lo_cells(T.ls) * kCellDoubles;
-            if (T.in_smem)
+            if (T.cells && T.in_smem)
+                gravity_columns<NT>(smem_dyn, order, j0, j1, px, py, pz, a);
+            else if (T.cells)
+                gravity_columns<NT>(gtab, order, j0, j1, px, py, pz, a);
+            else if (T.in_smem)
                 gravity_columns_split<NT>(smem_dyn, reinterpret_cast<const float*>(smem_dyn + lo_doubles), order, T.ls,
                                           j0, j1, px, py, pz, a);
             else
@@ -544,7 +550,7 @@ inline GravLaunch gravity_launch(const GravTable& T, int64_t n, int sms, int thr
     if (threads < 32) threads = 32;
     G.threads = threads / 32 * 32;
     const int warps = G.threads / 32;
-    if (T.ls > 0) {
+    if (T.ls > 0 || T.cells) {
         G.form = kGravSplit;
         G.units = sms;
         for (G.aux = kGravityPartsMax;; G.aux = 1) {

@@ -1241,7 +1241,10 @@ __device__ __forceinline__ void cheb_eval_pair(double t, double* low, double* mi
 }
 
 // fixed_fit: use the fixed-node sweep fits (c_fixed_fit) where they apply.
-template <int L>
+// A species' number density is fac exp(off); kLn carries ln fac + off instead,
+// in density()'s order: five logarithms more, the same to the last bits of ln
+// fac.
+template <int L, bool kLn>
 __device__ double density_group(const EpochR<double>& E, double sun_dec, double hour_angle, double lat, double alt_m,
                                 const Drivers& d, int q, unsigned gmask, bool fixed_fit,
                                 const JbFit2* fit2 = nullptr) {
@@ -1309,12 +1312,12 @@ __device__ double density_group(const EpochR<double>& E, double sun_dec, double 
     double fact2 = anm / 28.960;
     const double fac[5] = {JBT(kFrac)[0] * fact2, fact2 * (1.0 + JBT(kFrac)[1]) - an, 2.0 * (an - fact2),
                            JBT(kFrac)[2] * fact2, JBT(kFrac)[3] * fact2};
-    // a species' number density is fac exp(off) (density() carries ln fac
-    // instead: five logarithms more, the same to the last bits of ln fac)
     double off[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (kLn)
+        for (int i = 0; i < 5; ++i) off[i] = fac[i] < 0.0 ? NAN : log(fac[i]);
     double z = lo.z;
     if (alt <= 105.0) {
-        off[5] = -25.0;
+        off[5] = kLn ? off[4] - 25.0 : -25.0;
     } else {
         SweepG mid;
         if (use_fit && alt >= 500.0) {
@@ -1362,8 +1365,8 @@ __device__ double density_group(const EpochR<double>& E, double sun_dec, double 
             hsign = -1.0;
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) off[i] = -altr - fact2 * JBT(kAmw)[i];
-        off[4] = -(1.0 - 0.38) * altr - fact2 * JBT(kAmw)[4];
+        for (int i = 0; i < 4; ++i) off[i] = off[i] - altr - fact2 * JBT(kAmw)[i];
+        off[4] = off[4] - (1.0 - 0.38) * altr - fact2 * JBT(kAmw)[4];
         const double al10t5 = log10(tinf);
         const double alnh5 = (5.5 * al10t5 - 39.40) * al10t5 + 73.13;
         off[5] = kLn10 * (alnh5 + 6.0) + hsign * (log(tloc4 / tloc3) + up.sum * JBT(kAmw)[5] / kRstar);
@@ -1385,7 +1388,8 @@ __device__ double density_group(const EpochR<double>& E, double sun_dec, double 
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         const double f = i < 5 ? fac[i] : (alt <= 105.0 ? fac[4] : 1.0);
-        sumnm += (f < 0.0 ? NAN : f) * exp(off[i] + dlr) * JBT(kAmw)[i];
+        const double nd = exp(off[i] + dlr);
+        sumnm += (kLn ? nd : (f < 0.0 ? NAN : f) * nd) * JBT(kAmw)[i];
     }
     rho = sumnm / kAvogadro;
     double fex = 1.0;

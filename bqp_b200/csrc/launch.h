@@ -48,6 +48,14 @@ struct PropArgs {
     CtrlParams ctrl;
     const jb::JbFit* fit_host;     // host copy of *force.fit (null with it): the stage-synchronous
                                    // drag kernel takes it by value, in kernel parameter space
+    // Sigma-point rows in the GMST frame.  That frame's instant is a one-part
+    // Julian day, a 40 us staircase, and at tight tolerances an adaptive step's
+    // length follows the last bits of the force through it: rows then end
+    // 1e-8 km apart, which the covariance, made of the rows' differences, shows
+    // at 1e-9 of itself.  So for these rows the field and the density are added
+    // up in a fixed order of operations whatever kernel runs them: the cells'
+    // (GravTable::cells), and jb2008's with ln of each species (density()).
+    int32_t ordered;
     struct EclState* ecl;          // [n] eclipse coordinator state of SRP rows (null without SRP)
 };
 

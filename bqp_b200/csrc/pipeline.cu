@@ -439,7 +439,9 @@ __global__ void __launch_bounds__(kBlock) pl_sur_check(PipeBufs P, int cur, doub
 // [0, nb_hi) take list 0 with LH lanes per state, the rest list 1 with LL),
 // so that a stage's states are resident together in as few waves as the
 // register budget allows.
-// kForm 0: the exact model; 1, 2: the coarse profiles in FP64 and in FP32.
+// kForm 0: the exact model; 1, 2: the coarse profiles in FP64 and in FP32; 3:
+// the exact model in the order of PropArgs::ordered (and the profiles without
+// the fixed plans' ends: plan null).
 template <int L, int kForm = 0>
 __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs& P, int st, int list, int block) {
     const int gt = block * blockDim.x + threadIdx.x;
@@ -474,8 +476,9 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
             // same verdict on every lane of the group
             if (isnan(E.tsubc))
                 rho = NAN;
-            else if (kForm == 0)
-                rho = jb::density_group<L>(E, dec, ha, lat, alt_m, dr, q, gmask, fp.fit != nullptr, fp.fit2);
+            else if (kForm == 0 || kForm == 3)
+                rho = jb::density_group<L, kForm == 3>(E, dec, ha, lat, alt_m, dr, q, gmask, fp.fit != nullptr,
+                                                       fp.fit2);
             else if (!jb::geometry_valid(dec, ha, lat, alt_m))
                 rho = NAN;
             else if (kForm == 2)
@@ -517,10 +520,10 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
         for (int i = 0; i < 3; ++i) P.adrag[(size_t)i * P.cap + slot] = a[i];
 }
 
-template <int LH, int LL, int kMinBlocks>
+template <int LH, int LL, int kMinBlocks, int kForm>
 __global__ void __launch_bounds__(kDragBlock, kMinBlocks) pl_drag(ForceParams fp, PipeBufs P, int st, int nb_hi) {
-    if ((int)blockIdx.x < nb_hi) drag_rows<LH>(fp, P, st, 0, blockIdx.x);
-    else drag_rows<LL>(fp, P, st, 1, blockIdx.x - nb_hi);
+    if ((int)blockIdx.x < nb_hi) drag_rows<LH, kForm>(fp, P, st, 0, blockIdx.x);
+    else drag_rows<LL, kForm>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
 // The coarse profiles (atm_model 5-7): a short chain per state, one lane
@@ -734,8 +737,9 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     const int dblocks_hi = (int)((A.n * kLanesHigh + kDragBlock - 1) / kDragBlock);
     const int dblocks_lo = (int)((A.n * kLanesLow + kDragBlock - 1) / kDragBlock);
     // more registers a thread while a stage's rows still fit in one wave
-    auto dker = dblocks_hi <= 2 * device_sm_count() ? pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS_FEW>
-                                                    : pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS>;
+    auto dker = A.ordered ? pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS_FEW, 3>
+                : dblocks_hi <= 2 * device_sm_count() ? pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS_FEW, 0>
+                                                      : pl_drag<kLanesHigh, kLanesLow, BQP_DRAG_MIN_BLOCKS, 0>;
     const int cblocks = (int)((A.n + kDragBlock - 1) / kDragBlock);
     // with the surrogate, the exact stage covers only the degrees it leaves out
     const bool sur = A.sur.P != nullptr;
@@ -746,7 +750,7 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     // half of the registers to the drag kernel, and four warps of four rows a
     // lane still keep the FP64 pipe as busy as the table reads let it: 65,536
     // rows 331 ms a pass against 398 with 256 threads, 20,001 rows 179 and 210
-    if (A.force.drag && !times && gthreads == 256) gthreads = 128;
+    if (A.force.drag && !times && gthreads == 256 && !A.ordered) gthreads = 128;
     GravLaunch G = gravity_launch(GT, A.n, device_sm_count(), gthreads, gslots);
     GravLaunch GF = check ? gravity_launch(A.sur.full, A.n, device_sm_count(), gthreads, gslots) : G;
     auto gker = pl_gravity_of(G), gker_full = pl_gravity_of(GF);
