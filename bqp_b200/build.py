@@ -11,15 +11,16 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "_lib"
 LIB = LIB_DIR / "libbqp_b200.so"
-SOURCES = ["propagate.cu", "pipeline.cu", "eclipse.cu", "sigma.cu", "mlp.cu", "surrogate.cu", "space_weather.cu", "ephemeris.cu",
+SOURCES = ["attempt.cu", "propagate.cu", "pipeline.cu", "eclipse.cu", "sigma.cu", "mlp.cu", "surrogate.cu", "space_weather.cu", "ephemeris.cu",
            "bqp_api.cu", "frame_time.cpp"]
-HEADERS = ["kernels.cuh", "gravity.cuh", "gravity_cta.cuh", "jb2008.cuh", "physics.cuh", "launch.h", "rk_tableaus.h",
+HEADERS = ["kernels.cuh", "stages.cuh", "replay.h", "gravity.cuh", "gravity_cta.cuh", "jb2008.cuh", "physics.cuh", "launch.h", "rk_tableaus.h",
            "traj.cuh", "eclipse.cuh", "tc_gemm.cuh", "space_weather.h", "ephemeris.h", "surrogate.h",
            "frame_time.h", "frame_time_host.h", "iau2000a_tables.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -44,22 +45,25 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and not _stale():
         return LIB
     LIB_DIR.mkdir(exist_ok=True)
-    objs = []
     flags = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", *ARCH,
              "-I", str(CSRC), "-I", str(PKG.parent / "include")]
     # extra nvcc definitions for measured build variants (e.g. -DBQP_DRAG_MIN_BLOCKS=4)
     flags += os.environ.get("BQP_NVCC_DEFINES", "").split()
     if verbose:
         flags += ["-Xptxas", "-v"]
-    for src in SOURCES:
+
+    def compile_one(src: str) -> str:
         obj = LIB_DIR / (Path(src).stem + ".o")
-        cmd = [nvcc(), *flags, "-c", str(CSRC / src), "-o", str(obj)]
-        r = subprocess.run(cmd, capture_output=True, text=True)
+        r = subprocess.run([nvcc(), *flags, "-c", str(CSRC / src), "-o", str(obj)], capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed on {src}:\n{r.stderr}")
         if verbose and r.stderr:
             print(r.stderr, file=sys.stderr)
-        objs.append(str(obj))
+        return str(obj)
+
+    # the stage and attempt kernels take minutes each: side by side
+    with ThreadPoolExecutor(os.cpu_count() or 1) as pool:
+        objs = list(pool.map(compile_one, SOURCES))
     tmp = LIB.with_suffix(".so.tmp")
     cmd = [nvcc(), *ARCH, "-shared", "--cudart", "static", "-o", str(tmp), *objs]
     r = subprocess.run(cmd, capture_output=True, text=True)

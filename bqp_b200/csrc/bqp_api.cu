@@ -532,7 +532,7 @@ struct bqp_ctx {
     Coeffs coeffs;
     int parsed_order = 0;
     double* d_tab = nullptr;
-    double* d_tab_cells = nullptr;  // the same field as cells (sigma points in the GMST frame)
+    double* d_tab_cells = nullptr;  // the same field as cells (sigma points)
     int ncells = 0;
     size_t tab_bytes = 0;
     int use_smem = 0;
@@ -981,7 +981,7 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
     A.fit_host = A.force.fit ? &ctx->h_fit : nullptr;
     A.ctrl = ctrl_params(ctx);
     A.grav = grav_table(ctx);
-    if (sigma && A.force.frame.mode == 0 && A.grav.ls == 0 && !ctx->cfg.surrogate) {
+    if (sigma && A.grav.ls == 0 && !ctx->cfg.surrogate) {
         A.ordered = 1;
         A.force.plan.valid = 0;
         if (int rc = cells_table(ctx, A.grav)) return rc;

@@ -301,8 +301,8 @@ BQP_HD int gravity_part_column(int order, int p, int parts) {
 // The FP64 field with V and W both carried down every column and both
 // multiplied by their weights in every cell (12 operations a cell), over the
 // columns [j0, j1) of a table of cells {a, b, Ax, Bx, Ay, By, Az, Bz}.  Only
-// sigma-point rows in the GMST frame take it (PropArgs::ordered), for the
-// order in which it adds.
+// sigma-point rows take it (PropArgs::ordered), for the order in which it
+// adds.
 template <int NT>
 BQP_HD void gravity_columns(const double* __restrict__ tab, int order, int j0, int j1, const double* px,
                             const double* py, const double* pz, double (*acc)[3]) {

@@ -48,12 +48,12 @@ struct PropArgs {
     CtrlParams ctrl;
     const jb::JbFit* fit_host;     // host copy of *force.fit (null with it): the stage-synchronous
                                    // drag kernel takes it by value, in kernel parameter space
-    // Sigma-point rows in the GMST frame.  That frame's instant is a one-part
-    // Julian day, a 40 us staircase, and at tight tolerances an adaptive step's
-    // length follows the last bits of the force through it: rows then end
-    // 1e-8 km apart, which the covariance, made of the rows' differences, shows
-    // at 1e-9 of itself.  So for these rows the field and the density are added
-    // up in a fixed order of operations whatever kernel runs them: the cells'
+    // Sigma-point rows.  At tight tolerances an adaptive step's length follows
+    // the last bits of the force (in the GMST frame through its instant too, a
+    // one-part Julian day of 40 us steps): rows then end up to 1e-8 km apart,
+    // which the covariance, made of the rows' differences, shows at up to 2e-9
+    // of itself.  So for these rows the field and the density are added up in a
+    // fixed order of operations whatever kernel runs them: the cells'
     // (GravTable::cells), and jb2008's with ln of each species (density()).
     int32_t ordered;
     struct EclState* ecl;          // [n] eclipse coordinator state of SRP rows (null without SRP)
@@ -69,7 +69,7 @@ struct PipeBufs {
     int64_t cap;          // slots (= trajectories)
     TrajState* st;        // [cap]
     int32_t* idx[2];      // active lists (slot -> trajectory), double-buffered
-    int32_t* count;       // [2] active counts
+    int32_t* count;       // [2] active counts (attempt kernel: [3])
     double* k;            // [(S+1)][6][cap] stage derivatives
     double* sp;           // [6][cap] perturbed state of the stage (ECI)
     // what a stage needs of its instant alone, formed for several stages at
@@ -106,6 +106,13 @@ void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau, int drag);
 cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st,
                             double max_seconds, int gravity_threads, int gravity_slots,
                             KernelTimes* times = nullptr);
+
+// The stage kernels' preparation of all stages' instants (pipeline.cu), for the
+// rows of idx[list] counted in count[counter].
+void launch_times(const PropArgs& A, const PipeBufs& P, int method, int list, int counter, int stages, cudaStream_t st);
+// The attempt kernel (attempt.cu): whether it takes this batch, and its run.
+bool attempt_fits(const PropArgs& A, int method);
+cudaError_t launch_attempts(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st, double max_seconds);
 
 cudaError_t launch_gravity(const GravTable& T, int64_t n, const double* pos, double* acc, int32_t* status,
                            cudaStream_t st, int threads = 256, int slots = 4);
