@@ -119,7 +119,7 @@ __device__ __forceinline__ void attempt_gravity_cells(const PipeBufs& P, const G
 
 }  // namespace
 
-// Attempt number `at` of the graph: rows of list at % 2, counted in
+// Attempt number `at` of six: rows of list at % 2, counted in
 // count[at % 3]; rows that go on are appended to the other list and
 // count[(at + 1) % 3], and count[(at + 2) % 3] is cleared for the launch after
 // this one (nothing reads it any more).
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
 }
 
 template <int M>
-static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, double max_seconds) {
+static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaStream_t user, double max_seconds) {
     const bool dense = (A.out_mode != kOutFinalEci || A.force.srp) && !Tab<M>::FSAL;
     const int shares = kAttemptThreads / 32 - (A.force.drag ? kDragWarps : 0);
     const size_t smem = attempt_smem_bytes(A.grav, shares);
@@ -223,7 +223,7 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     const int blocks = (int)((A.n + kBlock - 1) / kBlock);
     const int ctas = (int)(A.n < device_sm_count() ? A.n : device_sm_count());
     return replay(
-        A, P, user, max_seconds, false, [&](cudaStream_t st) { pl_init<M><<<blocks, kBlock, 0, st>>>(A, P); },
+        P, R, user, max_seconds, false, false, [&](cudaStream_t st) { pl_init<M><<<blocks, kBlock, 0, st>>>(A, P); },
         [&](cudaStream_t st, cudaStream_t, const StreamOrder&) {
             // six attempts bring the two lists and the three counters back
             for (int at = 0; at < 6; ++at) {
@@ -240,13 +240,14 @@ bool attempt_fits(const PropArgs& A, int method) {
     return !A.force.gravity_on || attempt_smem_bytes(A.grav, kAttemptThreads / 32) <= kAttemptSmem;
 }
 
-cudaError_t launch_attempts(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st, double max_seconds) {
+cudaError_t launch_attempts(const PropArgs& A, const PipeBufs& P, ReplayRes& R, int method, cudaStream_t st,
+                            double max_seconds) {
     switch (method) {
-        case kDopri5: return run<kDopri5>(A, P, st, max_seconds);
-        case kDop853: return run<kDop853>(A, P, st, max_seconds);
-        case kDopri5Compat: return run<kDopri5Compat>(A, P, st, max_seconds);
-        case kVern7: return run<kVern7>(A, P, st, max_seconds);
-        case kVern9: return run<kVern9>(A, P, st, max_seconds);
+        case kDopri5: return run<kDopri5>(A, P, R, st, max_seconds);
+        case kDop853: return run<kDop853>(A, P, R, st, max_seconds);
+        case kDopri5Compat: return run<kDopri5Compat>(A, P, R, st, max_seconds);
+        case kVern7: return run<kVern7>(A, P, R, st, max_seconds);
+        case kVern9: return run<kVern9>(A, P, R, st, max_seconds);
         default: return cudaErrorInvalidValue;
     }
 }

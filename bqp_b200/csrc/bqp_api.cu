@@ -543,6 +543,7 @@ struct bqp_ctx {
     void* d_ws = nullptr;
     size_t ws_bytes = 0;
     void* d_pws = nullptr;  // stage-synchronous engine buffers
+    ReplayRes replay;       // and its host loop's streams and events
     size_t pws_bytes = 0;
     jb::JbFit* d_fit = nullptr;  // JB2008 fixed-node sweep fits (device)
     double fit_worst = -1.0;
@@ -1019,7 +1020,7 @@ int launch_prop(bqp_ctx* ctx, int64_t n, const double* in, int32_t input_equ, co
         }
         PipeBufs P{};
         pipeline_carve(P, ctx->d_pws, n, iau, A.force.drag);
-        cudaError_t e = launch_pipeline(A, P, ctx->cfg.method, ctx->stream, ctx->cfg.max_kernel_seconds,
+        cudaError_t e = launch_pipeline(A, P, ctx->replay, ctx->cfg.method, ctx->stream, ctx->cfg.max_kernel_seconds,
                                         ctx->cfg.gravity_threads, ctx->cfg.gravity_slots,
                                         ctx->profile ? &ctx->times : nullptr);
         if (e != cudaSuccess) return cuda_fail(e, "pipeline");
@@ -1297,6 +1298,7 @@ int bqp_ctx_destroy(bqp_ctx* ctx) {
     if (ctx->d_ecl) cudaFree(ctx->d_ecl);
     if (ctx->d_ws) cudaFree(ctx->d_ws);
     if (ctx->d_pws) cudaFree(ctx->d_pws);
+    ctx->replay.release();
     if (ctx->d_fit) cudaFree(ctx->d_fit);
     if (ctx->d_tab_split) cudaFree(ctx->d_tab_split);
     if (ctx->d_fit2) cudaFree(ctx->d_fit2);

@@ -101,9 +101,20 @@ struct KernelTimes {
     int64_t launches[kKcCount];
 };
 
+// The host loop's streams, events and pinned count (replay.h), kept by the
+// context: made at its first propagation, given back with it.  Creating and
+// destroying them, and a graph for six launches, took 2 ms of a call.
+struct ReplayRes {
+    cudaStream_t st = nullptr, st2 = nullptr;
+    cudaEvent_t ev_in = nullptr, ev_out = nullptr, ev_cnt = nullptr, ev_order = nullptr;
+    int32_t* h_count = nullptr;
+    cudaError_t ready();
+    void release();
+};
+
 size_t pipeline_bytes(int64_t cap, int iau, int drag);
 void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau, int drag);
-cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st,
+cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, ReplayRes& R, int method, cudaStream_t st,
                             double max_seconds, int gravity_threads, int gravity_slots,
                             KernelTimes* times = nullptr);
 
@@ -112,7 +123,8 @@ cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cu
 void launch_times(const PropArgs& A, const PipeBufs& P, int method, int list, int counter, int stages, cudaStream_t st);
 // The attempt kernel (attempt.cu): whether it takes this batch, and its run.
 bool attempt_fits(const PropArgs& A, int method);
-cudaError_t launch_attempts(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st, double max_seconds);
+cudaError_t launch_attempts(const PropArgs& A, const PipeBufs& P, ReplayRes& R, int method, cudaStream_t st,
+                            double max_seconds);
 
 cudaError_t launch_gravity(const GravTable& T, int64_t n, const double* pos, double* acc, int32_t* status,
                            cudaStream_t st, int threads = 256, int slots = 4);

@@ -308,8 +308,30 @@ void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau, int drag) {
     P.dcount = (int32_t*)take(2 * (size_t)P.ring * 4);  // last: pipeline_bytes measures up to it
 }
 
+cudaError_t ReplayRes::ready() {
+    if (h_count) return cudaSuccess;
+    int low = 0, high = 0;
+    cudaDeviceGetStreamPriorityRange(&low, &high);
+    cudaError_t e = cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, high);
+    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, low);
+    for (cudaEvent_t* ev : {&ev_in, &ev_out, &ev_cnt, &ev_order})
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMallocHost(&h_count, sizeof(int32_t));
+    if (e != cudaSuccess) release();
+    return e;
+}
+
+void ReplayRes::release() {
+    if (h_count) cudaFreeHost(h_count);
+    for (cudaEvent_t ev : {ev_in, ev_out, ev_cnt, ev_order})
+        if (ev) cudaEventDestroy(ev);
+    if (st2) cudaStreamDestroy(st2);
+    if (st) cudaStreamDestroy(st);
+    *this = ReplayRes{};
+}
+
 template <int M>
-static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, double max_seconds,
+static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaStream_t user, double max_seconds,
                        int gthreads, int gslots, KernelTimes* times) {
     using T = Tab<M>;
     // the dense stage: the end-of-step derivative of sampled segments and of
@@ -427,7 +449,7 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
         }
     };
     e = replay(
-        A, P, user, max_seconds, times != nullptr,
+        P, R, user, max_seconds, true, times != nullptr,
         [&](cudaStream_t st) {
             if (check) cudaMemsetAsync(P.fall, 0, (size_t)A.n * sizeof(int32_t), st);
             pl_init<M><<<blocks, kBlock, 0, st>>>(A, P);
@@ -442,19 +464,20 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, cudaStream_t user, 
     return e;
 }
 
-cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, int method, cudaStream_t st, double max_seconds,
+cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, ReplayRes& R, int method, cudaStream_t st,
+                            double max_seconds,
                             int gravity_threads, int gravity_slots, KernelTimes* times) {
     if (A.n <= 0) return cudaSuccess;
     if (gravity_threads <= 0) gravity_threads = 256;
     if (!times && gravity_threads == 256 && gravity_slots != 1 && gravity_slots != 2 && attempt_fits(A, method))
-        return launch_attempts(A, P, method, st, max_seconds);
+        return launch_attempts(A, P, R, method, st, max_seconds);
     switch (method) {
-        case kDopri5: return run<kDopri5>(A, P, st, max_seconds, gravity_threads, gravity_slots, times);
-        case kDop853: return run<kDop853>(A, P, st, max_seconds, gravity_threads, gravity_slots, times);
+        case kDopri5: return run<kDopri5>(A, P, R, st, max_seconds, gravity_threads, gravity_slots, times);
+        case kDop853: return run<kDop853>(A, P, R, st, max_seconds, gravity_threads, gravity_slots, times);
         case kDopri5Compat:
-            return run<kDopri5Compat>(A, P, st, max_seconds, gravity_threads, gravity_slots, times);
-        case kVern7: return run<kVern7>(A, P, st, max_seconds, gravity_threads, gravity_slots, times);
-        case kVern9: return run<kVern9>(A, P, st, max_seconds, gravity_threads, gravity_slots, times);
+            return run<kDopri5Compat>(A, P, R, st, max_seconds, gravity_threads, gravity_slots, times);
+        case kVern7: return run<kVern7>(A, P, R, st, max_seconds, gravity_threads, gravity_slots, times);
+        case kVern9: return run<kVern9>(A, P, R, st, max_seconds, gravity_threads, gravity_slots, times);
         default: return cudaErrorInvalidValue;
     }
 }

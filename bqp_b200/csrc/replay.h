@@ -1,5 +1,5 @@
-// Host loop of the stage-synchronous engine: a graph of attempts, captured
-// once a call and replayed until no row is active.
+// Host loop of the stage-synchronous engine: attempts issued until no row is
+// active.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -30,68 +30,62 @@ struct StreamOrder {
     }
 };
 
-// init(st) fills the first active list; enqueue(st, st2, order) captures the
-// graph, after which list 0 and count[0] are the active rows again; abort(st)
-// ends the rows of list 0.  timed: collect() reads each replay's events.
+// init(st) fills the first active list; enqueue(st, st2, order) issues some
+// attempts, after which list 0 and count[0] are the active rows again --
+// captured once as a graph and replayed (`graph`), or launched as they are (a
+// few launches: cheaper than to instantiate a graph a call); abort(st) ends
+// the rows of list 0.  timed: collect() reads each replay's events.
 template <class Init, class Enqueue, class Abort, class Collect>
-static cudaError_t replay(const PropArgs& A, const PipeBufs& P, cudaStream_t user, double max_seconds, bool timed,
-                          Init init, Enqueue enqueue, Abort abort, Collect collect) {
-    (void)A;
-    // private stream ordered after the caller's stream (graphs need a
-    // capturable stream), and a second one, whose kernels give way to the
-    // first's
-    int prio_low = 0, prio_high = 0;
-    cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
-    cudaStream_t st, st2;
-    cudaError_t e = cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, prio_high);
+static cudaError_t replay(const PipeBufs& P, ReplayRes& R, cudaStream_t user, double max_seconds, bool graph_on,
+                          bool timed, Init init, Enqueue enqueue, Abort abort, Collect collect) {
+    // streams of the context's own, ordered after the caller's (graphs need a
+    // capturable stream); the second one's kernels give way to the first's
+    cudaError_t e = R.ready();
     if (e != cudaSuccess) return e;
-    e = cudaStreamCreateWithPriority(&st2, cudaStreamNonBlocking, prio_low);
-    if (e != cudaSuccess) {
-        cudaStreamDestroy(st);
-        return e;
-    }
-    cudaEvent_t ev_in, ev_out, ev_cnt, ev_order;
-    cudaEventCreateWithFlags(&ev_in, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&ev_out, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&ev_cnt, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&ev_order, cudaEventDisableTiming);
-    cudaEventRecord(ev_in, user);
-    cudaStreamWaitEvent(st, ev_in, 0);
-    int32_t* h_count = nullptr;
-    cudaMallocHost(&h_count, sizeof(int32_t));
+    const cudaStream_t st = R.st, st2 = R.st2;
+    const StreamOrder order{R.ev_order};
+    cudaEventRecord(R.ev_in, user);
+    cudaStreamWaitEvent(st, R.ev_in, 0);
 
     cudaMemsetAsync(P.count, 0, 3 * sizeof(int32_t), st);
     init(st);
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        enqueue(st, st2, StreamOrder{ev_order});
-        e = cudaStreamEndCapture(st, &graph);
+    if (graph_on) {
+        e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            enqueue(st, st2, order);
+            e = cudaStreamEndCapture(st, &graph);
+        }
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
+    auto issue = [&]() -> cudaError_t {
+        if (graph_on) return cudaGraphLaunch(exec, st);
+        enqueue(st, st2, order);
+        return cudaGetLastError();
+    };
     const auto t_start = std::chrono::steady_clock::now();
     // host loop: replay, keep one replay in flight ahead of the count check
     bool done = false;
     while (e == cudaSuccess && !done) {
-        e = cudaGraphLaunch(exec, st);
+        e = issue();
         if (e != cudaSuccess) break;
-        cudaMemcpyAsync(h_count, &P.count[0], sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-        cudaEventRecord(ev_cnt, st);
+        cudaMemcpyAsync(R.h_count, &P.count[0], sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+        cudaEventRecord(R.ev_cnt, st);
         if (timed) {
             // no replay in flight while the events of this one are read
-            e = cudaEventSynchronize(ev_cnt);
+            e = cudaEventSynchronize(R.ev_cnt);
             if (e != cudaSuccess) break;
             collect();
         }
-        e = cudaGraphLaunch(exec, st);  // speculative: cheap when nothing is active
+        e = issue();  // speculative: cheap when nothing is active
         if (e != cudaSuccess) break;
-        e = cudaEventSynchronize(ev_cnt);
+        e = cudaEventSynchronize(R.ev_cnt);
         if (timed && e == cudaSuccess) {
             e = cudaStreamSynchronize(st);
             if (e == cudaSuccess) collect();
         }
-        if (*h_count == 0) done = true;
+        if (*R.h_count == 0) done = true;
         const double elapsed =
             std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
         if (!done && max_seconds > 0.0 && elapsed > max_seconds) {
@@ -101,18 +95,11 @@ static cudaError_t replay(const PropArgs& A, const PipeBufs& P, cudaStream_t use
         }
     }
     if (e == cudaSuccess) e = cudaGetLastError();
-    cudaEventRecord(ev_out, st);
-    cudaStreamWaitEvent(user, ev_out, 0);
+    cudaEventRecord(R.ev_out, st);
+    cudaStreamWaitEvent(user, R.ev_out, 0);
     cudaStreamSynchronize(st);
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
-    cudaFreeHost(h_count);
-    cudaEventDestroy(ev_in);
-    cudaEventDestroy(ev_out);
-    cudaEventDestroy(ev_cnt);
-    cudaEventDestroy(ev_order);
-    cudaStreamDestroy(st2);
-    cudaStreamDestroy(st);
     return e;
 }
 
