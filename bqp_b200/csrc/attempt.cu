@@ -194,6 +194,8 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
                 attempt_drag<4, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
             else if (fp.atm_model == 4)
                 attempt_drag<2, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+            else if (wide && !fp.drag_fp32 && !A.ordered)
+                attempt_drag<4, 4>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
             else if (fp.drag_fp32)
                 attempt_drag<1, 2>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
             else

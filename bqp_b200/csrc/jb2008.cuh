@@ -1408,6 +1408,211 @@ __device__ double density_group(const EpochR<double>& E, double sun_dec, double 
     if (!(isfinite(out) && out > 0.0)) return kErrDomain;
     return out;
 }
+
+// ------------------------------------------------------------------------
+// density_coarse_core<double> by a group of four lanes (q = lane within the
+// group, gmask = the group's lanes; same inputs in every lane, which branch
+// together).  The chain is the profile's; calls of one function that do not
+// depend on one another are one call on different lanes: the four sines and
+// cosines of the exospheric temperature, a panel's four nodes, the closing
+// logarithms, the species' exponentials.  About 10 long calls follow one
+// another instead of 25, and the code a warp fetches shrinks alike.
+// One panel after the other, node j + 1 of each on lane j.
+__device__ __forceinline__ SweepR<double> boole_sweep_quad(double z, double zend_start, double zr, int n, double ain,
+                                                           bool with_mbar, const double* tc, int q, unsigned gmask) {
+    SweepR<double> s;
+    s.sum = 0.0;
+    s.zend = zend_start;
+    s.z = z;
+    s.tloc = s.gravl = s.mb = 0.0;
+    const double w = q == 0 || q == 2 ? kW1 : (q == 1 ? kW2 : kW0);
+    for (int i = 0; i < n; ++i) {
+        const double z0 = s.zend;
+        s.zend = zr * z0;
+        const double dz = 0.25 * (s.zend - z0);
+        const double z1 = z0 + dz, z2 = z1 + dz, z3 = z2 + dz, z4 = z3 + dz;  // as the walk adds them
+        const double zz = q == 0 ? z1 : q == 1 ? z2 : q == 2 ? z3 : z4;
+        s.tloc = local_temp_r(zz, tc);
+        s.gravl = grav_r(zz);
+        s.mb = with_mbar ? mbar_r(zz) : 1.0;
+        const double a = with_mbar ? s.mb * s.gravl / s.tloc : s.gravl / s.tloc;
+        double sum1 = w * a;
+        sum1 += __shfl_xor_sync(gmask, sum1, 1, 4);
+        sum1 += __shfl_xor_sync(gmask, sum1, 2, 4);
+        s.sum += dz * (kW0 * ain + sum1);
+        ain = __shfl_sync(gmask, a, 3, 4);
+        s.z = z4;
+    }
+    s.tloc = __shfl_sync(gmask, s.tloc, 3, 4);
+    s.gravl = __shfl_sync(gmask, s.gravl, 3, 4);
+    s.mb = __shfl_sync(gmask, s.mb, 3, 4);
+    s.ain = ain;
+    return s;
+}
+
+__device__ __forceinline__ double density_coarse_quad(const EpochR<double>& E, double sun_dec, double hour_angle,
+                                                      double lat, double alt_m, const Drivers& d, int model,
+                                                      const CoarsePlan* plan, int q, unsigned gmask) {
+    const double step_lower = 0.040, step_middle = model == 5 ? 0.100 : 0.300;
+    const double step_upper = model == 5 ? 0.300 : 0.700;
+    const bool v7 = model == 7;
+    const double alt = alt_m / 1000.0;
+    double h = hour_angle;
+    if (!(h >= 0.0 && h < kTwoPi)) {
+        if (h < 0.0 && h > -kTwoPi) {
+            h += kTwoPi;
+        } else {
+            h = fmod(h, kTwoPi);
+            if (h < 0.0) h += kTwoPi;
+        }
+    }
+    const double eta = 0.5 * fabs(lat - sun_dec), theta = 0.5 * fabs(lat + sun_dec);
+    double sq, cq;
+    sincos(q == 0 ? h + 0.75049158 : q == 1 ? lat : q == 2 ? eta : theta, &sq, &cq);
+    const double tau = h - 0.64577182 + 0.10471976 * __shfl_sync(gmask, sq, 0, 4);
+    const double slat = __shfl_sync(gmask, sq, 1, 4), clat = __shfl_sync(gmask, cq, 1, 4);
+    const double ce = __shfl_sync(gmask, cq, 2, 4), sn = __shfl_sync(gmask, sq, 3, 4);
+    double st_hour = ((h + kPi) * (180.0 / kPi)) / 15.0;
+    if (st_hour >= 24.0) st_hour -= 24.0;
+    else if (st_hour < 0.0) st_hour += 24.0;
+    const double root = sqrt(q & 1 ? sn : ce);
+    const double cos_eta = ce * ce * __shfl_sync(gmask, root, 0, 4);
+    const double sin_theta = sn * sn * __shfl_sync(gmask, root, 1, 4);
+    const double cos_tau = fabs(cos(0.5 * tau));
+    const double df = sin_theta + (cos_eta - sin_theta) * cos_tau * cos_tau * cos_tau;
+    const double tsubl = E.tsubc * (1.0 + 0.31 * df);
+    const double tinf = tsubl + d.dtc + dtc_correction_r(d.f10, st_hour, clat, alt);
+    const double hm90 = alt - 90.0;
+    const double eq = exp(q & 1 ? -0.045 * hm90 : -0.0021357 * tinf);
+    const double tsubx = 444.3807 + 0.02385 * tinf - 392.8292 * __shfl_sync(gmask, eq, 0, 4);
+    const double exp_h = __shfl_sync(gmask, eq, 1, 4);
+    const double gsubx = 0.054285714 * (tsubx - 183.0);
+    double tc[4];
+    tc[0] = tsubx;
+    tc[1] = gsubx;
+    tc[2] = (tinf - tsubx) / (kPi / 2);
+    tc[3] = gsubx / tc[2];
+    const double texo = tc[0] + tc[2] * (kPi / 2);
+    const bool fit_in = v7 && texo >= kV7TexoLo && texo <= kV7TexoHi;
+    const double u = 2.0 * (texo - kV7TexoLo) / (kV7TexoHi - kV7TexoLo) - 1.0;
+    const double z1 = 90.0;
+    const double mb1 = mbar_r(z1);
+    const double tloc1 = local_temp_r(z1, tc);
+    const bool lower_planned = alt >= 105.0;
+    const bool planned = fit_in && lower_planned && plan && plan->valid;
+    double al;
+    int n;
+    SweepR<double> lo;
+    if (planned) {
+        lo.mb = plan->low_mb;
+        lo.gravl = plan->low_gravl;
+        lo.z = plan->low_z;
+        lo.zend = plan->low_zend;
+    } else {
+        al = log(fmin(alt, 105.0) / z1);
+        n = coarse_panels(al / step_lower);
+        if (n == 0) return kErrDomain;
+        lo = boole_sweep_quad(z1, z1, exp(al / n), n, mb1 * grav_r(z1) / tloc1, true, tc, q, gmask);
+    }
+    if (fit_in && lower_planned) {
+        lo.sum = v7_series(JBT(kV7Sub2Lower), u);
+        lo.tloc = v7_series(JBT(kV7Tloc2), u);
+    }
+    const double mb2 = lo.mb, tloc2 = lo.tloc;
+    double rho = 3.46e-6 * mb2 * tloc1 / exp(lo.sum / kRstar) / (mb1 * tloc2);
+    const double anm = kAvogadro * rho;
+    const double an = anm / mb2;
+    double fact2 = anm / 28.960;
+    double factor[6] = {JBT(kFrac)[0] * fact2, fact2 * (1.0 + JBT(kFrac)[1]) - an, 2.0 * (an - fact2),
+                        JBT(kFrac)[2] * fact2, JBT(kFrac)[3] * fact2, 1.0};
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+        if (factor[i] < 0.0) factor[i] = NAN;
+    double offset[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double z = lo.z;
+    if (alt <= 105.0) {
+        factor[5] = factor[4];
+        offset[5] = offset[4] - 25.0;
+    } else {
+        SweepR<double> mid;
+        if (planned && alt >= 500.0) {
+            mid.z = plan->mid_z;
+            mid.zend = plan->mid_zend;
+        } else {
+            al = log(fmin(alt, 500.0) / z);
+            n = coarse_panels(al / step_middle);
+            if (n == 0) return kErrDomain;
+            mid = boole_sweep_quad(z, lo.zend, exp(al / n), n, lo.gravl / tloc2, false, tc, q, gmask);
+        }
+        if (fit_in && lower_planned && alt >= 500.0) {
+            mid.sum = v7_series(JBT(kV7Sub2Middle), u);
+            mid.ain = v7_series(JBT(kV7AinMiddle), u);
+            mid.tloc = v7_series(JBT(kV7Tloc3), u);
+        }
+        const double tloc3 = mid.tloc;
+        z = mid.z;
+        const double ratio = fmax(alt, 500.0) / z;
+        const double alu = fmax(log(ratio), 0.0);
+        n = coarse_panels(alu / (alt > 500.0 ? step_upper : step_middle));
+        if (n == 0) return kErrDomain;
+        const double zr = (v7 && n == 1) ? fmax(ratio, 1.0) : exp(alu / n);
+        const SweepR<double> up = boole_sweep_quad(z, mid.zend, zr, n, mid.ain, false, tc, q, gmask);
+        const double tloc4 = up.tloc;
+        z = up.z;
+        const bool low = alt <= 500.0;
+        const double lq = log(q == 0 ? (low ? tloc3 : tloc4) / tloc2 : q == 1 ? tloc4 / tloc3 : tinf);
+        const double altr = __shfl_sync(gmask, lq, 0, 4);
+        const double al10t5 = __shfl_sync(gmask, lq, 2, 4) / kLn10;
+        fact2 = (low ? mid.sum : mid.sum + up.sum) / kRstar;
+        const double hsign = low ? 1.0 : -1.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) offset[i] = offset[i] - altr - fact2 * JBT(kAmw)[i];
+        offset[4] = offset[4] - (1.0 - 0.38) * altr - fact2 * JBT(kAmw)[4];
+        const double alnh5 = (5.5 * al10t5 - 39.40) * al10t5 + 73.13;
+        offset[5] = kLn10 * (alnh5 + 6.0) + hsign * (__shfl_sync(gmask, lq, 1, 4) + up.sum * JBT(kAmw)[5] / kRstar);
+    }
+    double dlrsl = 0.0;
+    if (!(v7 && alt >= 800.0)) dlrsl = 0.02 * hm90 * exp_h * (lat >= 0.0 ? 1.0 : -1.0) * E.sinphi * slat * slat;
+    double dlrsa = 0.0;
+    if (z < 2000.0) {
+        if (isnan(E.gtz)) return kErrDomain;  // the day is out of range
+        const double htz = alt / 1000.0;
+        const double fz = d.f10b - 0.70 * d.s10b - 0.04 * d.m10b;
+        const double fzz = JBT(kFzm)[0] + fz * (JBT(kFzm)[1] + htz * (JBT(kFzm)[2] + JBT(kFzm)[3] * htz + JBT(kFzm)[4] * fz));
+        dlrsa = fmax(fzz, 1.0e-6) * E.gtz;
+    }
+    const double dlr = kLn10 * (dlrsl + dlrsa);
+    // species 0..3, then 4 and 5; the compensated sum in their order
+    const double e0 = exp((q == 0 ? offset[0] : q == 1 ? offset[1] : q == 2 ? offset[2] : offset[3]) + dlr);
+    const double e1 = exp((q & 1 ? offset[5] : offset[4]) + dlr);
+    double sum = 0.0, comp = 0.0, simple = 0.0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+        const double ex = __shfl_sync(gmask, i < 4 ? e0 : e1, i & 3, 4);
+        const double term = factor[i] * ex * JBT(kAmw)[i];
+        const double tmp = term - comp;
+        const double next = sum + tmp;
+        comp = (next - sum) - tmp;
+        sum = next;
+        simple += term;
+    }
+    double fs = sum - comp;
+    if (isnan(fs) && isinf(simple)) fs = simple;
+    rho = fs / kAvogadro;
+    double fex = 1.0;
+    if (alt >= 1000.0 && alt < 1500.0) {
+        const double zeta = (alt - 1000.0) * 0.002;
+        const double f15c = JBT(kCht)[0] + JBT(kCht)[1] * d.f10b + JBT(kCht)[2] * 1500.0 +
+                            JBT(kCht)[3] * d.f10b * 1500.0;
+        const double f15cz = (JBT(kCht)[2] + JBT(kCht)[3] * d.f10b) * 500.0;
+        fex = 1.0 + zeta * zeta * ((3.0 * f15c - f15cz - 3.0) + (f15cz - 2.0 * f15c + 2.0) * zeta);
+    } else if (alt >= 1500.0) {
+        fex = JBT(kCht)[0] + JBT(kCht)[1] * d.f10b + JBT(kCht)[2] * alt + JBT(kCht)[3] * d.f10b * alt;
+    }
+    const double out = rho * fex;
+    if (!(isfinite(out) && out > 0.0)) return kErrDomain;
+    return out;
+}
 #endif  // __CUDACC__
 
 }  // namespace jb

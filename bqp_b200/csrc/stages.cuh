@@ -284,7 +284,8 @@ __device__ __forceinline__ bool prep_row(const PropArgs& A, const PipeBufs& P, c
 // gmask the group's lanes): the JB2008 model is the longest serial chain of the
 // force call, and it is bound by that latency, not by throughput.
 // kForm 0: the exact model; 1, 2: the coarse profiles in FP64 and in FP32; 3:
-// the exact model in the order of PropArgs::ordered.
+// the exact model in the order of PropArgs::ordered; 4: the coarse profiles in
+// FP64 by four lanes.
 template <int L, int kForm>
 __device__ __forceinline__ void drag_row(const ForceParams& fp, const PipeBufs& P, int st, int slot, int q,
                                          unsigned gmask) {
@@ -305,8 +306,17 @@ __device__ __forceinline__ void drag_row(const ForceParams& fp, const PipeBufs& 
             const double si0 = Q.drag(P, 0, slot), si1 = Q.drag(P, 1, slot), dec = Q.drag(P, 2, slot);
             const jb::EpochR<double> E{Q.drag(P, 3, slot), Q.drag(P, 4, slot), Q.drag(P, 5, slot)};
             const double alt_m = geodetic_altitude_km(pi[0], pi[1], pi[2], fp.earth_radius) * 1000.0;
-            const double ha = atan2(fma(pi[1], si0, -(pi[0] * si1)), fma(pi[0], si0, pi[1] * si1));
-            const double lat = asin(fmin(1.0, fmax(-1.0, pi[2] / sat_r)));
+            const double hy = fma(pi[1], si0, -(pi[0] * si1)), hx = fma(pi[0], si0, pi[1] * si1);
+            double ha, lat;
+            if (kForm == 4) {
+                // both angles in one call, on lanes 0 and 1
+                const double v = atan2(q & 1 ? pi[2] : hy, q & 1 ? sqrt(fma(pi[0], pi[0], pi[1] * pi[1])) : hx);
+                ha = __shfl_sync(gmask, v, 0, 4);
+                lat = __shfl_sync(gmask, v, 1, 4);
+            } else {
+                ha = atan2(hy, hx);
+                lat = asin(fmin(1.0, fmax(-1.0, pi[2] / sat_r)));
+            }
             jb::Drivers dr = fp.drivers;
             if (fp.dtab.n_solar > 0) jb::lookup_drivers(fp.dtab, Q.jd(slot), &dr);
             // fixed-node fits from constant memory (fp.fit holds the same numbers);
@@ -319,6 +329,8 @@ __device__ __forceinline__ void drag_row(const ForceParams& fp, const PipeBufs& 
                                                        fp.fit2);
             else if (!jb::geometry_valid(dec, ha, lat, alt_m))
                 rho = NAN;
+            else if (kForm == 4)
+                rho = jb::density_coarse_quad(E, dec, ha, lat, alt_m, dr, fp.atm_model, &fp.plan, q, gmask);
             else if (kForm == 2)
                 rho = jb::density_coarse_core<float>({(float)E.tsubc, (float)E.sinphi, (float)E.gtz}, dec, ha, lat,
                                                      alt_m, dr, fp.atm_model, &fp.plan);
