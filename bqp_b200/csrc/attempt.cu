@@ -1,15 +1,15 @@
-// Attempt kernel: a whole step attempt of a small batch in one launch.
+// Attempt kernel: whole step attempts of a small batch in one launch.
 //
 // With a few thousand rows the stage kernels (pipeline.cu) are bound by what
 // each costs whatever its rows: a launch and its gap, the staging of the field
 // table, and one row's serial chain, three kernels a stage one after the other.
 // Trajectories do not depend on one another, so here a CTA keeps a few rows
-// (at most kAttemptRows) through all stages of the attempt: the instants'
+// (at most kAttemptRows) through all stages of its attempts: the instants'
 // chains of all stages run side by side first (one part of one stage of one
 // row a thread), then stage by stage a thread a row prepares, and four warps
 // evaluate the drag (up to four lanes a row) while the others share the field's
-// columns; the controller closes the attempt.  The table is staged once an
-// attempt, under the instants' chains.  The field's sums are added in the order
+// columns; the controller closes the attempt.  The table is staged once a
+// launch, under the first attempt's instants.  The field's sums are added in the order
 // of the shares, the same for every batch.
 //
 // us a pass, stage kernels -> attempt kernel: one satellite over an hour, every
@@ -33,6 +33,11 @@ namespace {
 constexpr int kAttemptThreads = 384, kDragWarps = 4;
 // rows a CTA keeps: two tiles of a warp, the controller's two warps
 constexpr int kAttemptRows = 64;
+// Attempts a CTA makes on its rows before the rows that go on are dealt out
+// again.  CTAs then wait for one another once a launch, not once an attempt:
+// with SRP a row that crosses the shadow's edge keeps its CTA's controller for
+// most of a millisecond, a few rows of 1,500 in every attempt.
+constexpr int kAttemptRounds = 16;
 
 // the table and the shares' sums, beside the static arrays
 constexpr size_t kAttemptSmem = 227 * 1024 - 12 * 1024;
@@ -119,24 +124,28 @@ __device__ __forceinline__ void attempt_gravity_cells(const PipeBufs& P, const G
 
 }  // namespace
 
-// Attempt number `at` of six: rows of list at % 2, counted in
-// count[at % 3]; rows that go on are appended to the other list and
+// Launch number `at` of six: up to `rounds` attempts of the rows of list at % 2,
+// counted in count[at % 3]; rows that go on are appended to the other list and
 // count[(at + 1) % 3], and count[(at + 2) % 3] is cleared for the launch after
 // this one (nothing reads it any more).
 template <int M>
 __global__ void __launch_bounds__(kAttemptThreads, 1)
-    at_attempt(const __grid_constant__ PropArgs A, const __grid_constant__ PipeBufs P, int at, int dense) {
+    at_attempt(const __grid_constant__ PropArgs A, const __grid_constant__ PipeBufs P, int at, int dense,
+               int rounds) {
     extern __shared__ __align__(16) double smem_dyn[];  // [shares][3][kAttemptRows] sums, the table
     __shared__ __align__(8) uint64_t bar;
     __shared__ EclWarpStore ecl_ws[kAttemptRows / 32];
     // drag: rows above and below ~510 km; the counts of this stage and the next
     __shared__ int32_t n_list[2][2], row_list[2][kAttemptRows];
+    // the CTA's trajectories, of this attempt and the next; row r is slot b0 + r
+    __shared__ int32_t trajs[2][kAttemptRows], n_traj[2];
     const int count = P.count[at % 3];
     const int per = (count + gridDim.x - 1) / gridDim.x;
-    const int b0 = blockIdx.x * per, rows = min(per, count - b0);
+    const int b0 = blockIdx.x * per;
+    int rows = min(per, count - b0);
     if (blockIdx.x == 0 && threadIdx.x == 0) P.count[(at + 2) % 3] = 0;
     if (rows <= 0) return;  // uniform across the CTA
-    const int32_t* list = P.idx[at & 1];
+    if (threadIdx.x < rows) trajs[0][threadIdx.x] = P.idx[at & 1][b0 + threadIdx.x];
     const ForceParams& fp = A.force;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int drag_warps = fp.drag ? kDragWarps : 0;
@@ -147,71 +156,83 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
     if (fp.gravity_on)
         staged = stage_begin(&bar, A.grav.bytes, [&](auto copy) { copy(tab, A.grav.tab, A.grav.bytes); });
     const int stages = Tab<M>::S + (dense ? 1 : 0);
-    // the instants: part k of stage s of row r, the parts in different warps
-    // (ordered rows: pl_times has run)
-    if (!A.ordered) {
-        const int items = rows * stages, padded = (items + 31) & ~31;
-        for (int i = tid; i < 4 * padded; i += kAttemptThreads) {
-            const int part = i / padded, k = i - part * padded;
-            if (k >= items) continue;
-            const int st = k / rows, slot = b0 + k - st * rows;
-            const TrajState& s = P.st[list[slot]];
-            if (st == 0 && (s.flags & kHaveK1)) continue;
-            times_row(A, P, s, slot, st, stage_time<M>(s, st), 1 << part);
+    __syncthreads();  // the trajectories are listed
+    int round = 0;
+    for (; round < rounds && rows > 0; ++round) {
+        const int32_t* list = trajs[round & 1];
+        if (tid == 0) n_traj[(round & 1) ^ 1] = 0;  // read again after the stages' barriers
+        // the instants: part k of stage s of row r, the parts in different warps
+        // (ordered rows: pl_times has run)
+        if (!A.ordered) {
+            const int items = rows * stages, padded = (items + 31) & ~31;
+            for (int i = tid; i < 4 * padded; i += kAttemptThreads) {
+                const int part = i / padded, k = i - part * padded;
+                if (k >= items) continue;
+                const int st = k / rows, slot = b0 + k - st * rows;
+                const TrajState& s = P.st[list[slot - b0]];
+                if (st == 0 && (s.flags & kHaveK1)) continue;
+                times_row(A, P, s, slot, st, stage_time<M>(s, st), 1 << part);
+            }
         }
-    }
-    if (fp.gravity_on && staged) staged = stage_wait(&bar);
-    for (int st = 0; st <= stages; ++st) {
-        if (st == 0 && tid < 2) n_list[0][tid] = 0;
-        __syncthreads();  // the last stage's sums and drag are there
-        if (tid < 2) n_list[(st + 1) & 1][tid] = 0;
-        if (tid < rows) {
-            const int slot = b0 + tid;
-            if (st > 0 && fp.gravity_on && !P.skip[slot]) {
-                const int sums = A.grav.cells ? kGravityPartsMax : shares;
-                for (int k = 0; k < 3; ++k) {
-                    double g = red[k * kAttemptRows + tid];
-                    for (int w = 1; w < sums; ++w) g += red[(w * 3 + k) * kAttemptRows + tid];
-                    P.agrav[(size_t)k * P.cap + slot] = g;
+        if (round == 0 && fp.gravity_on && staged) staged = stage_wait(&bar);
+        for (int st = 0; st <= stages; ++st) {
+            if (st == 0 && tid < 2) n_list[0][tid] = 0;
+            __syncthreads();  // the last stage's sums and drag are there
+            if (tid < 2) n_list[(st + 1) & 1][tid] = 0;
+            if (tid < rows) {
+                const int slot = b0 + tid;
+                if (st > 0 && fp.gravity_on && !P.skip[slot]) {
+                    const int sums = A.grav.cells ? kGravityPartsMax : shares;
+                    for (int k = 0; k < 3; ++k) {
+                        double g = red[k * kAttemptRows + tid];
+                        for (int w = 1; w < sums; ++w) g += red[(w * 3 + k) * kAttemptRows + tid];
+                        P.agrav[(size_t)k * P.cap + slot] = g;
+                    }
+                }
+                double r2;
+                if (st < stages && prep_row<M>(A, P, P.st[list[slot - b0]], slot, st, &r2) && fp.drag) {
+                    const int c = sqrt(r2) - fp.earth_radius >= 510.0 ? 0 : 1;
+                    row_list[c][atomicAdd(&n_list[st & 1][c], 1)] = tid;
                 }
             }
-            double r2;
-            if (st < stages && prep_row<M>(A, P, P.st[list[slot]], slot, st, &r2) && fp.drag) {
-                const int c = sqrt(r2) - fp.earth_radius >= 510.0 ? 0 : 1;
-                row_list[c][atomicAdd(&n_list[st & 1][c], 1)] = tid;
+            if (st == stages) break;
+            __syncthreads();
+            if (warp < drag_warps) {
+                const int hi = n_list[st & 1][0], lo = n_list[st & 1][1];
+                const bool wide = (hi + 7) / 8 + (lo + 7) / 8 <= kDragWarps;  // four lanes a row in one pass
+                if (fp.atm_model == 4 && A.ordered) {
+                    // as the stage kernels' lanes: one a row above, four below
+                    attempt_drag<1, 3>(fp, P, st, b0, row_list[0], hi, row_list[1], 0);
+                    attempt_drag<4, 3>(fp, P, st, b0, row_list[0], 0, row_list[1], lo);
+                } else if (fp.atm_model == 4 && wide)
+                    attempt_drag<4, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+                else if (fp.atm_model == 4)
+                    attempt_drag<2, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+                else if (wide && !fp.drag_fp32 && !A.ordered)
+                    attempt_drag<4, 4>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+                else if (fp.drag_fp32)
+                    attempt_drag<1, 2>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+                else
+                    attempt_drag<1, 1>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+            } else if (fp.gravity_on) {
+                if (A.grav.cells)
+                    attempt_gravity_cells(P, A.grav, tab, st, b0, rows, warp - drag_warps, staged, red);
+                else if (rows <= 32)
+                    attempt_gravity<1>(P, A.grav, tab, st, b0, rows, shares, warp - drag_warps, staged, red);
+                else
+                    attempt_gravity<2>(P, A.grav, tab, st, b0, rows, shares, warp - drag_warps, staged, red);
             }
         }
-        if (st == stages) break;
+        if (warp * 32 < rows)
+            control_warp<M>(A, P, tid < rows ? list[tid] : 0, b0 + tid, tid < rows, trajs[(round & 1) ^ 1],
+                            &n_traj[(round & 1) ^ 1], ecl_ws[warp], dense);
         __syncthreads();
-        if (warp < drag_warps) {
-            const int hi = n_list[st & 1][0], lo = n_list[st & 1][1];
-            const bool wide = (hi + 7) / 8 + (lo + 7) / 8 <= kDragWarps;  // four lanes a row in one pass
-            if (fp.atm_model == 4 && A.ordered) {
-                // as the stage kernels' lanes: one a row above, four below
-                attempt_drag<1, 3>(fp, P, st, b0, row_list[0], hi, row_list[1], 0);
-                attempt_drag<4, 3>(fp, P, st, b0, row_list[0], 0, row_list[1], lo);
-            } else if (fp.atm_model == 4 && wide)
-                attempt_drag<4, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-            else if (fp.atm_model == 4)
-                attempt_drag<2, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-            else if (wide && !fp.drag_fp32 && !A.ordered)
-                attempt_drag<4, 4>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-            else if (fp.drag_fp32)
-                attempt_drag<1, 2>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-            else
-                attempt_drag<1, 1>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-        } else if (fp.gravity_on) {
-            if (A.grav.cells)
-                attempt_gravity_cells(P, A.grav, tab, st, b0, rows, warp - drag_warps, staged, red);
-            else if (rows <= 32)
-                attempt_gravity<1>(P, A.grav, tab, st, b0, rows, shares, warp - drag_warps, staged, red);
-            else
-                attempt_gravity<2>(P, A.grav, tab, st, b0, rows, shares, warp - drag_warps, staged, red);
-        }
+        rows = n_traj[(round & 1) ^ 1];
     }
-    if (warp * 32 < rows)
-        control_warp<M>(A, P, list, b0 + tid, tid < rows, P.idx[(at & 1) ^ 1], &P.count[(at + 1) % 3], ecl_ws[warp],
-                        dense);
+    if (tid < rows) {
+        const int i = atomicAdd(&P.count[(at + 1) % 3], 1);
+        P.idx[(at & 1) ^ 1][i] = trajs[round & 1][tid];
+    }
 }
 
 template <int M>
@@ -230,7 +251,8 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
             // six attempts bring the two lists and the three counters back
             for (int at = 0; at < 6; ++at) {
                 if (A.ordered) launch_times(A, P, M, at & 1, at % 3, Tab<M>::S + (dense ? 1 : 0), st);
-                at_attempt<M><<<ctas, kAttemptThreads, smem, st>>>(A, P, at, dense ? 1 : 0);
+                at_attempt<M><<<ctas, kAttemptThreads, smem, st>>>(A, P, at, dense ? 1 : 0,
+                                                                  A.ordered ? 1 : kAttemptRounds);
             }
         },
         [&](cudaStream_t st) { pl_abort<M><<<blocks, kBlock, 0, st>>>(A, P, 0); }, [] {});

@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(kBlock) pl_control(const __grid_constant__ Pro
     const int slot = blockIdx.x * blockDim.x + threadIdx.x;
     const int count = P.count[cur];
     if (slot - (int)(threadIdx.x & 31) >= count) return;  // the whole warp is idle
-    control_warp<M>(A, P, P.idx[cur], slot, slot < count, P.idx[cur ^ 1], &P.count[cur ^ 1],
+    control_warp<M>(A, P, slot < count ? P.idx[cur][slot] : 0, slot, slot < count, P.idx[cur ^ 1], &P.count[cur ^ 1],
                     ecl_ws[threadIdx.x >> 5], dense);
 }
 

@@ -379,23 +379,21 @@ __device__ __forceinline__ void drag_row(const ForceParams& fp, const PipeBufs& 
 constexpr int64_t kEclSoloSplits = BQP_ECL_SOLO_SPLITS;
 
 // The end of an attempt for the 32 rows of a warp (all lanes take part; row
-// `slot` of `list` where active): the last stage, the error, accept or reject,
+// `traj` in slot `slot` where active): the last stage, the error, accept or reject,
 // samples, rectification, the next attempt; rows that go on are appended to
 // `next`.  ws: the warp's store for the cooperative eclipse scan (SRP rows).
 template <int M>
-__device__ __forceinline__ void control_warp(const PropArgs& A, const PipeBufs& P, const int32_t* list, int slot,
+__device__ __forceinline__ void control_warp(const PropArgs& A, const PipeBufs& P, int32_t traj, int slot,
                                              bool active, int32_t* next, int32_t* next_count, EclWarpStore& ws,
                                              int dense) {
     using T = Tab<M>;
     const int lane = threadIdx.x & 31;
     bool keep = false;
-    int32_t traj = 0;
     TrajState s;
     bool scan = false;  // an accepted SRP step waiting for its crossing scan
     EclScanReq req;
     double tn = 0.0, en = 0.0, ynext[6], k0[6], dyn[6];
     if (active) {
-        traj = list[slot];
         s = P.st[traj];
         const int last = dense ? T::S : T::S - 1;
         if (!(last == 1 && P.skip[slot])) finish_stage(P, last, slot);

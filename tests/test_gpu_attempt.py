@@ -5,7 +5,11 @@ to the stage kernels.  A gravity_threads other than the default keeps a batch
 on the stage kernels.
 
 Tolerance: two adaptive solutions of the same equations, each within
-10 eps a step of the exact one (as the engines' comparison with the oracle).
+10 eps a step of the exact one (as the engines' comparison with the oracle),
+which holds where the force is smooth on the scale of a step.  Without the
+field (order 0) steps grow to dt_max and JB2008's branches in altitude (its
+local-time correction ends at 800 km) set the difference of any two solutions,
+so that case is checked where the rows take the same bits: sigma points.
 """
 import numpy as np
 import pytest
@@ -42,7 +46,6 @@ def context(order, method, atm, flags, frame="gmst", stages=False, fp32=False):
     (64 * SMS, 6, "dopri5_solver", 6, 4, "gmst", 300.0, True),
     (64 * SMS + 1, 6, "vern7", 7, 4, "gmst", 300.0, False),
     (300, 78, "dop853", 4, 4 | 8, "iau2006", 600.0, False),
-    (300, 0, "vern9", 4, 4 | 8, "gmst", 6000.0, False),
     (65, 12, "vern7", 7, 2 | 4 | 8, "iau2006", 6000.0, False),
 ])
 def test_attempt_kernel_against_the_stage_kernels(n, order, method, atm, flags, frame, arc, fp32):
@@ -76,12 +79,13 @@ def test_sampled_rows_and_failures():
     assert dr.max() <= 2e-5  # interior samples: the Hermite interpolant's own error
 
 
-@pytest.mark.parametrize("atm,frame", [(0, "gmst"), (4, "gmst"), (7, "gmst"), (4, "iau2006"), (7, "iau2006")])
-def test_sigma_points_take_the_same_bits(atm, frame):
+@pytest.mark.parametrize("order,atm,frame", [(20, 0, "gmst"), (20, 4, "gmst"), (20, 7, "gmst"), (20, 4, "iau2006"),
+                                             (20, 7, "iau2006"), (0, 4, "gmst"), (0, 7, "iau2006")])
+def test_sigma_points_take_the_same_bits(order, atm, frame):
     """Kernels timed by class run as stage kernels; the rows keep their order
     of operations in both."""
     mean, cov = workloads.ukf_objects(90, seed=4)
-    ctx = context(20, "dop853", atm, 4 | 8, frame)
+    ctx = context(order, "dop853", atm, 4 | 8, frame)
     a = ctx.sigma_propagate(mean, cov, workloads.EPOCH_JD, 3000.0)
     ctx.profile(True)
     b = ctx.sigma_propagate(mean, cov, workloads.EPOCH_JD, 3000.0)
