@@ -153,6 +153,11 @@ int device_sm_count();
 // out[i * si + k * sk] (surrogate.cu).  Grid sized for up to cap rows.
 cudaError_t launch_surrogate_stage(const SurrogateRef& S, const int32_t* n_dev, int64_t cap, const double* pos,
                                    double* out, int64_t si, int64_t sk, cudaStream_t st);
+// The same with the reduction over K split over CTAs, for products of few
+// tiles; part: kGemmSplitsMax M N floats; C 16-byte aligned.
+constexpr int kGemmSplitsMax = 32;
+cudaError_t launch_gemm_bf16_split(int64_t M, int64_t N, int64_t K, const void* A, const void* B, float* C,
+                                   float* part, int* err, cudaStream_t st);
 cudaError_t launch_gemm_bf16(int64_t M, int64_t N, int64_t K, const void* A, const void* B, float* C, int* err,
                              cudaStream_t st);
 

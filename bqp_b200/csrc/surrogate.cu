@@ -203,50 +203,77 @@ __global__ void k_transpose(int rows, int cols, const __nv_bfloat16* __restrict_
     }
 }
 
-// column sums of a [B][cols] BF16 matrix (bias gradients); one block per column
-__global__ void k_colsum(int B, int cols, const __nv_bfloat16* __restrict__ m, float* __restrict__ out) {
-    __shared__ float part[256];
-    const int c = blockIdx.x;
-    float s = 0.0f;
-    for (int b = threadIdx.x; b < B; b += blockDim.x) s += __bfloat162float(m[(size_t)b * cols + c]);
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[c] = part[0];
+// Sums over the batch, a block a run of kGradRows rows, a thread a column (rows
+// are read whole; a block a column read 32 bytes for every 2): partial sums of
+// width values, added by k_grad_sums.  Four running sums a value.
+constexpr int kGradRows = 64;
+
+// column sums of a [B][256] BF16 matrix (bias gradients)
+__global__ void __launch_bounds__(kH) k_col_partials(const __nv_bfloat16* __restrict__ m, float* __restrict__ part) {
+    const __nv_bfloat16* r = m + (size_t)blockIdx.x * kGradRows * kH + threadIdx.x;
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 4
+    for (int b = 0; b < kGradRows; b += 4)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s[q] += __bfloat162float(r[(size_t)(b + q) * kH]);
+    part[(size_t)blockIdx.x * kH + threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
 }
 
-// output and input layer weight gradients (small reductions over the batch)
-__global__ void k_small_grads(int B, const float* __restrict__ dy, const __nv_bfloat16* __restrict__ h3,
-                              const __nv_bfloat16* __restrict__ dz0, const float* __restrict__ xb,
-                              float* __restrict__ G) {
-    __shared__ float part[256];
-    // blocks 0..767: dW4[k][j]; 768..770: db4[k]; 771..1794: dW0[j][k]
-    const int id = blockIdx.x;
-    float s = 0.0f;
-    if (id < 3 * kH) {
-        const int k = id / kH, j = id % kH;
-        for (int b = threadIdx.x; b < B; b += blockDim.x) s += dy[3 * b + k] * __bfloat162float(h3[(size_t)b * kH + j]);
-    } else if (id < 3 * kH + 3) {
-        const int k = id - 3 * kH;
-        for (int b = threadIdx.x; b < B; b += blockDim.x) s += dy[3 * b + k];
-    } else {
-        const int q = id - 3 * kH - 3, j = q / 4, k = q % 4;
-        for (int b = threadIdx.x; b < B; b += blockDim.x) s += __bfloat162float(dz0[(size_t)b * kH + j]) * xb[4 * b + k];
+// the output and input layers' gradients: dW4[k][j], dW0[j][k], db0[j], db4[k]
+constexpr int kEdgeWidth = 8 * kH + 4;
+__global__ void __launch_bounds__(kH)
+    k_edge_partials(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ h3,
+                    const __nv_bfloat16* __restrict__ dz0, const float* __restrict__ xb, float* __restrict__ part) {
+    const int j = threadIdx.x;
+    const size_t b0 = (size_t)blockIdx.x * kGradRows;
+    float s[4][8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[q][k] = 0.0f;
+    for (int b = 0; b < kGradRows; b += 4)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const size_t r = b0 + b + q;
+            const float h = __bfloat162float(h3[r * kH + j]), z = __bfloat162float(dz0[r * kH + j]);
+            const float4 x = *reinterpret_cast<const float4*>(xb + 4 * r);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) s[q][k] = fmaf(dy[3 * r + k], h, s[q][k]);
+            s[q][3] = fmaf(z, x.x, s[q][3]);
+            s[q][4] = fmaf(z, x.y, s[q][4]);
+            s[q][5] = fmaf(z, x.z, s[q][5]);
+            s[q][6] = fmaf(z, x.w, s[q][6]);
+            s[q][7] += z;
+        }
+    float* p = part + (size_t)blockIdx.x * kEdgeWidth;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k * kH + j] = (s[0][k] + s[1][k]) + (s[2][k] + s[3][k]);
+    if (j < 4) {
+        float d = 0.0f;
+        if (j < 3)
+            for (int b = 0; b < kGradRows; ++b) d += dy[3 * (b0 + b) + j];
+        p[8 * kH + j] = d;
     }
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        if (id < 3 * kH) G[kOffW4 + id] = part[0];
-        else if (id < 3 * kH + 3) G[kOffB4 + id - 3 * kH] = part[0];
-        else G[kOffW0 + id - 3 * kH - 3] = part[0];
-    }
+}
+
+// G[place of value i] = sum of the blocks' partial sums i (edge: k_edge_partials'
+// values; else consecutive from `off`)
+__global__ void k_grad_sums(int blocks, int width, const float* __restrict__ part, float* __restrict__ G, int off,
+                            bool edge) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= width) return;
+    float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    for (int b = 0; b < blocks; b += 8)
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (b + q < blocks) s[q] += part[(size_t)(b + q) * width + i];
+    const float v = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+    const int k = i / kH, j = i - k * kH;
+    if (!edge) G[off + i] = v;
+    else if (k < 3) G[kOffW4 + i] = v;
+    else if (k < 7) G[kOffW0 + j * 4 + (k - 3)] = v;
+    else if (k == 7) G[kOffB0 + j] = v;
+    else if (j < 3) G[kOffB4 + j] = v;
 }
 
 // Adam on the FP32 masters; refresh the BF16 copies of the hidden layers
@@ -511,10 +538,10 @@ Model::~Model() { release(); }
 void Model::release() {
     // dsum points into derr and is not freed on its own
     void* ptrs[] = {P, G, m1, m2, W, Wt, Wtile, x, t, xb, tb, z[0], z[1], z[2], z[3], h[0], h[1], h[2], h[3], dz[0], dz[1],
-                    dz[2], dz[3], dzt, ht, dh, y, dy, derr};
+                    dz[2], dz[3], dzt, ht, dh, y, dy, wpart, gpart, derr};
     for (void* p : ptrs)
         if (p) cudaFree(p);
-    P = G = m1 = m2 = x = t = xb = tb = dh = y = dy = nullptr;
+    P = G = m1 = m2 = x = t = xb = tb = dh = y = dy = wpart = gpart = nullptr;
     W = Wt = Wtile = dzt = ht = nullptr;
     for (int l = 0; l < 4; ++l) {
         z[l] = nullptr;
@@ -544,7 +571,8 @@ cudaError_t Model::alloc_params() {
 
 cudaError_t Model::alloc_batch(int B) {
     if (B <= batch_cap) return cudaSuccess;
-    void* ptrs[] = {xb, tb, z[0], z[1], z[2], z[3], h[0], h[1], h[2], h[3], dz[0], dz[1], dz[2], dz[3], dzt, ht, dh, y, dy};
+    void* ptrs[] = {xb, tb, z[0], z[1], z[2], z[3], h[0], h[1], h[2], h[3], dz[0], dz[1], dz[2], dz[3], dzt, ht, dh, y, dy,
+                    wpart, gpart};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     xb = tb = nullptr;
@@ -554,7 +582,7 @@ cudaError_t Model::alloc_batch(int B) {
         dz[l] = nullptr;
     }
     dzt = ht = nullptr;
-    dh = y = dy = nullptr;
+    dh = y = dy = wpart = gpart = nullptr;
     cudaError_t e = cudaSuccess;
     auto A = [&](void** p, size_t bytes) {
         if (e == cudaSuccess) e = cudaMalloc(p, bytes);
@@ -572,6 +600,8 @@ cudaError_t Model::alloc_batch(int B) {
     A((void**)&dh, BH * 4);
     A((void**)&y, (size_t)B * 3 * 4);
     A((void**)&dy, (size_t)B * 3 * 4);
+    A((void**)&wpart, (size_t)kGemmSplitsMax * sg::kH * sg::kH * 4);
+    A((void**)&gpart, (size_t)(B / sg::kGradRows) * sg::kEdgeWidth * 4);
     if (e == cudaSuccess) batch_cap = B;
     return e;
 }
@@ -618,16 +648,18 @@ cudaError_t forward_backward(Model& M, int B, bool train, cudaStream_t st) {
         const dim3 tb(32, 8), tg((unsigned)(kH / 32), (unsigned)(B / 32));
         k_transpose<<<tg, tb, 0, st>>>(B, kH, M.dz[l], M.dzt);
         k_transpose<<<tg, tb, 0, st>>>(B, kH, M.h[l - 1], M.ht);
-        cudaError_t e = launch_gemm_bf16(kH, kH, B, M.dzt, M.ht, M.G + kOffW1 + (l - 1) * kH * kH, M.derr, st);
+        cudaError_t e = launch_gemm_bf16_split(kH, kH, B, M.dzt, M.ht, M.G + kOffW1 + (l - 1) * kH * kH, M.wpart,
+                                               M.derr, st);
         if (e != cudaSuccess) return e;
-        k_colsum<<<kH, 256, 0, st>>>(B, kH, M.dz[l], M.G + kOffB1 + (l - 1) * kH);
+        k_col_partials<<<B / kGradRows, kH, 0, st>>>(M.dz[l], M.gpart);
+        k_grad_sums<<<kH / 64, 64, 0, st>>>(B / kGradRows, kH, M.gpart, M.G, kOffB1 + (l - 1) * kH, false);
         // dH_{l-1} = dZ_l W_l:  A = dZ_l [B][H(out)], B_op = W_l^T [H(in)][H(out)]
         e = launch_gemm_bf16(B, kH, kH, M.dz[l], M.Wt + (size_t)(l - 1) * kH * kH, M.dh, M.derr, st);
         if (e != cudaSuccess) return e;
         k_silu_back<<<blocks_for(BH), 256, 0, st>>>(B, M.dh, M.z[l - 1], M.dz[l - 1]);
     }
-    k_colsum<<<kH, 256, 0, st>>>(B, kH, M.dz[0], M.G + kOffB0);
-    k_small_grads<<<3 * kH + 3 + 4 * kH, 256, 0, st>>>(B, M.dy, M.h[3], M.dz[0], M.xb, M.G);
+    k_edge_partials<<<B / kGradRows, kH, 0, st>>>(M.dy, M.h[3], M.dz[0], M.xb, M.gpart);
+    k_grad_sums<<<blocks_for(kEdgeWidth, 64), 64, 0, st>>>(B / kGradRows, kEdgeWidth, M.gpart, M.G, 0, true);
     return cudaGetLastError();
 }
 

@@ -54,6 +54,7 @@ struct Model {
     __nv_bfloat16* dz[4] = {nullptr, nullptr, nullptr, nullptr};
     __nv_bfloat16 *dzt = nullptr, *ht = nullptr;
     float *dh = nullptr, *y = nullptr, *dy = nullptr;
+    float *wpart = nullptr, *gpart = nullptr;  // partial sums of the weight and of the other gradients
     double* dsum = nullptr;
     int* derr = nullptr;  // [0] GEMM wait timeout, then sigma (double at +8), loss sum (double at +16)
 

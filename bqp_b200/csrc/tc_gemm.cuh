@@ -87,11 +87,12 @@ __device__ __forceinline__ void load_stage(const __nv_bfloat16* __restrict__ A, 
     }
 }
 
-// The tile loop.  epi(row, col0, v[16]) receives 16 consecutive FP32 results
-// of one row (col0 = first column of C).
+// The tile loop over k0 <= k < k1 (multiples of kBK; K: the operands' row
+// length).  epi(row, col0, v[16]) receives 16 consecutive FP32 results of one
+// row (col0 = first column of C).
 template <class Epilogue>
 __device__ __forceinline__ void gemm_tile(const __nv_bfloat16* __restrict__ A, const __nv_bfloat16* __restrict__ B,
-                                          int K, int m0, int n0, int* err, Epilogue epi) {
+                                          int K, int k0, int k1, int m0, int n0, int* err, Epilogue epi) {
     extern __shared__ __align__(128) unsigned char tc_smem[];
     __nv_bfloat16* sa[2] = {reinterpret_cast<__nv_bfloat16*>(tc_smem),
                             reinterpret_cast<__nv_bfloat16*>(tc_smem + kStageA + kStageB)};
@@ -120,7 +121,7 @@ __device__ __forceinline__ void gemm_tile(const __nv_bfloat16* __restrict__ A, c
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
 
-    const int nk = K / kBK;
+    const int nk = (k1 - k0) / kBK;
     uint32_t phase[2] = {0, 0};
     bool pending[2] = {false, false};  // a commit on this buffer's barrier not yet seen complete
     bool ok = true;
@@ -133,7 +134,7 @@ __device__ __forceinline__ void gemm_tile(const __nv_bfloat16* __restrict__ A, c
             phase[buf] ^= 1u;
             pending[buf] = false;
         }
-        load_stage(A, B, K, m0, n0, s * kBK, sa[buf], sb[buf]);
+        load_stage(A, B, K, m0, n0, k0 + s * kBK, sa[buf], sb[buf]);
         // make the generic-proxy stores visible to the tensor cores
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
