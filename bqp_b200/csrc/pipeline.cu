@@ -227,20 +227,25 @@ __device__ __forceinline__ void drag_rows(const ForceParams& fp, const PipeBufs&
 }
 
 template <int LH, int LL, int kMinBlocks, int kForm>
-__global__ void __launch_bounds__(kDragBlock, kMinBlocks) pl_drag(ForceParams fp, PipeBufs P, int st, int nb_hi) {
+__global__ void __launch_bounds__(kDragBlock, kMinBlocks) pl_drag(const __grid_constant__ ForceParams fp,
+                                                              const __grid_constant__ PipeBufs P, int st, int nb_hi) {
     if ((int)blockIdx.x < nb_hi) drag_rows<LH, kForm>(fp, P, st, 0, blockIdx.x);
     else drag_rows<LL, kForm>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
-// The coarse profiles (atm_model 5-7): a short chain per state, one lane
-// each, both altitude lists in one launch.
+// The coarse profiles (atm_model 5-7), both altitude lists in one launch: above
+// ~510 km a short chain per state on one lane; below, up to twelve panels one
+// after the other, so four lanes take a state there (a node of each panel a
+// lane).  20,001 rows, model 7: 152,141 us a pass, 178,363 with one lane in
+// both.
 #ifndef BQP_COARSE_MIN_BLOCKS
 #define BQP_COARSE_MIN_BLOCKS 4
 #endif
-template <int kForm>
-__global__ void __launch_bounds__(kDragBlock, BQP_COARSE_MIN_BLOCKS) pl_drag_coarse(ForceParams fp, PipeBufs P, int st, int nb_hi) {
+template <int LL, int kForm, int kFormLow>
+__global__ void __launch_bounds__(kDragBlock, BQP_COARSE_MIN_BLOCKS)
+    pl_drag_coarse(const __grid_constant__ ForceParams fp, const __grid_constant__ PipeBufs P, int st, int nb_hi) {
     if ((int)blockIdx.x < nb_hi) drag_rows<1, kForm>(fp, P, st, 0, blockIdx.x);
-    else drag_rows<1, kForm>(fp, P, st, 1, blockIdx.x - nb_hi);
+    else drag_rows<LL, kFormLow>(fp, P, st, 1, blockIdx.x - nb_hi);
 }
 
 // ------------------------------------------------------------------ control
@@ -429,9 +434,11 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
                     if (A.force.atm_model == 4)
                         dker<<<dblocks_hi + dblocks_lo, kDragBlock, 0, sd>>>(A.force, P, s, dblocks_hi);
                     else if (A.force.drag_fp32)
-                        pl_drag_coarse<2><<<2 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
+                        pl_drag_coarse<1, 2, 2><<<2 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
+                    else if (A.ordered)
+                        pl_drag_coarse<1, 1, 1><<<2 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
                     else
-                        pl_drag_coarse<1><<<2 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
+                        pl_drag_coarse<4, 1, 4><<<5 * cblocks, kDragBlock, 0, sd>>>(A.force, P, s, cblocks);
                 });
             if (beside) {
                 order_after(st2, st);
