@@ -7,7 +7,7 @@
 // (at most kAttemptRows) through all stages of its attempts: the instants'
 // chains of all stages run side by side first (one part of one stage of one
 // row a thread), then stage by stage a thread a row prepares, and four warps
-// evaluate the drag (up to four lanes a row) while the others share the field's
+// evaluate the drag (four or two lanes a row) while the others share the field's
 // columns; the controller closes the attempt.  The table is staged once a
 // launch, under the first attempt's instants.  The field's sums are added in the order
 // of the shares, the same for every batch.
@@ -38,6 +38,15 @@ constexpr int kAttemptRows = 64;
 // with SRP a row that crosses the shadow's edge keeps its CTA's controller for
 // most of a millisecond, a few rows of 1,500 in every attempt.
 constexpr int kAttemptRounds = 16;
+// Rows a CTA up to which the exact density takes four lanes a row, two beyond.
+// Up to 25 rows four fit in one pass of the drag's warps whatever share of them
+// is above ~510 km; 32 to 64 rows take 4 to 7 % less with two (64 rows, 20x20,
+// 600 s: 30,276 us against 32,288).  The forms do not give the same bits, so
+// the rows a CTA are the launch's, not a CTA's own: which rows share a CTA, and
+// how many of them are above, differs from run to run.  The coarse profiles
+// take four lanes at any count (48 rows a CTA, 20x20: 13,246 us; 14,395 with
+// one lane a row where four did not fit in one pass).
+constexpr int kFourLanesRows = 25;
 
 // the table and the shares' sums, beside the static arrays
 constexpr size_t kAttemptSmem = 227 * 1024 - 12 * 1024;
@@ -139,6 +148,7 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
     __shared__ int32_t n_list[2][2], row_list[2][kAttemptRows];
     // the CTA's trajectories, of this attempt and the next; row r is slot b0 + r
     __shared__ int32_t trajs[2][kAttemptRows], n_traj[2];
+    __shared__ int32_t four_lanes;  // exact density: the launch's rows a CTA are at most kFourLanesRows
     const int count = P.count[at % 3];
     const int per = (count + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * per;
@@ -147,6 +157,7 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
     if (rows <= 0) return;  // uniform across the CTA
     if (threadIdx.x < rows) trajs[0][threadIdx.x] = P.idx[at & 1][b0 + threadIdx.x];
     const ForceParams& fp = A.force;
+    if (threadIdx.x == 0) four_lanes = per <= kFourLanesRows;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int drag_warps = fp.drag ? kDragWarps : 0;
     const int shares = kAttemptThreads / 32 - drag_warps;
@@ -199,21 +210,20 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
             __syncthreads();
             if (warp < drag_warps) {
                 const int hi = n_list[st & 1][0], lo = n_list[st & 1][1];
-                const bool wide = (hi + 7) / 8 + (lo + 7) / 8 <= kDragWarps;  // four lanes a row in one pass
                 if (fp.atm_model == 4 && A.ordered) {
                     // as the stage kernels' lanes: one a row above, four below
                     attempt_drag<1, 3>(fp, P, st, b0, row_list[0], hi, row_list[1], 0);
                     attempt_drag<4, 3>(fp, P, st, b0, row_list[0], 0, row_list[1], lo);
-                } else if (fp.atm_model == 4 && wide)
+                } else if (fp.atm_model == 4 && four_lanes)
                     attempt_drag<4, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
                 else if (fp.atm_model == 4)
                     attempt_drag<2, 0>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-                else if (wide && !fp.drag_fp32 && !A.ordered)
-                    attempt_drag<4, 4>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
                 else if (fp.drag_fp32)
                     attempt_drag<1, 2>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
-                else
+                else if (A.ordered)
                     attempt_drag<1, 1>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
+                else
+                    attempt_drag<4, 4>(fp, P, st, b0, row_list[0], hi, row_list[1], lo);
             } else if (fp.gravity_on) {
                 if (A.grav.cells)
                     attempt_gravity_cells(P, A.grav, tab, st, b0, rows, warp - drag_warps, staged, red);
