@@ -48,8 +48,10 @@ constexpr int kAttemptRounds = 16;
 // one lane a row where four did not fit in one pass).
 constexpr int kFourLanesRows = 25;
 
-// the table and the shares' sums, beside the static arrays
-constexpr size_t kAttemptSmem = 227 * 1024 - 12 * 1024;
+// the table and the shares' sums, beside the static arrays (at_attempt's)
+constexpr size_t kAttemptStatic = 12 * 1024, kAttemptSmem = kSmemLimit - kAttemptStatic;
+static_assert(sizeof(uint64_t) + kAttemptRows / 32 * sizeof(EclWarpStore) + (4 * kAttemptRows + 7) * sizeof(int32_t) + 64 <=
+              kAttemptStatic);
 size_t attempt_smem_bytes(const GravTable& T, int shares) {
     return ((size_t)shares * 3 * kAttemptRows + kGravityTabPad) * sizeof(double) + T.bytes;
 }
@@ -250,7 +252,8 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
     const bool dense = (A.out_mode != kOutFinalEci || A.force.srp) && !Tab<M>::FSAL;
     const int shares = kAttemptThreads / 32 - (A.force.drag ? kDragWarps : 0);
     const size_t smem = attempt_smem_bytes(A.grav, shares);
-    cudaError_t e = cudaFuncSetAttribute(at_attempt<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(at_attempt<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAttemptSmem);
     if (e == cudaSuccess) e = upload_fixed_fit(A, user);
     if (e != cudaSuccess) return e;
     const int blocks = (int)((A.n + kBlock - 1) / kBlock);
@@ -268,8 +271,7 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
         [&](cudaStream_t st) { pl_abort<M><<<blocks, kBlock, 0, st>>>(A, P, 0); }, [] {});
 }
 
-bool attempt_fits(const PropArgs& A, int method) {
-    (void)method;
+bool attempt_fits(const PropArgs& A) {
     if (A.sur.P || A.grav.ls > 0 || A.n > (int64_t)kAttemptRows * device_sm_count()) return false;
     return !A.force.gravity_on || attempt_smem_bytes(A.grav, kAttemptThreads / 32) <= kAttemptSmem;
 }

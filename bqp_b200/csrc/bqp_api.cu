@@ -47,7 +47,6 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 constexpr int kMaxOrder = 128;
-constexpr size_t kSmemLimit = 227 * 1024;
 
 // Normalised coefficients, [n*(order+1) + m].
 struct Coeffs {

@@ -589,11 +589,13 @@ cudaError_t gravity_run(const GravLaunch& G, void (*ker)(Params...), int ctas, c
     return cudaLaunchKernelEx(&c, ker, Params(args)...);
 }
 
-// Readies a kernel for G: its shared memory and, for clusters, how many the
-// device holds at once (fewer than SMs / CTAs where a GPC's SMs do not divide).
+// Readies a kernel for G: its shared memory (the bound, see kSmemLimit) and,
+// for clusters, how many the device holds at once (fewer than SMs / CTAs where
+// a GPC's SMs do not divide).
 template <class... Params>
 cudaError_t gravity_ready(GravLaunch& G, void (*ker)(Params...)) {
-    cudaError_t e = cudaFuncSetAttribute(ker, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G.smem);
+    if (G.smem > kSmemPerBlock) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(ker, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemPerBlock);
     if (e != cudaSuccess || G.cluster == 1) return e;
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeClusterDimension;

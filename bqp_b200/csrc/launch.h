@@ -101,6 +101,13 @@ struct KernelTimes {
     int64_t launches[kKcCount];
 };
 
+// Shared memory a CTA may have, static and dynamic.  What a kernel may ask for
+// (cudaFuncAttributeMaxDynamicSharedMemorySize) belongs to the function, for
+// every context and thread of the process: each kernel is given the most any
+// call of it asks for, never one call's size, which a call with a smaller field
+// would lower under another thread's launches.
+constexpr size_t kSmemLimit = 227 * 1024;
+
 // The host loop's streams, events and pinned count (replay.h), kept by the
 // context: made at its first propagation, given back with it.  Creating and
 // destroying them, and a graph for six launches, took 2 ms of a call.
@@ -122,7 +129,7 @@ cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, ReplayRes& R, 
 // rows of idx[list] counted in count[counter].
 void launch_times(const PropArgs& A, const PipeBufs& P, int method, int list, int counter, int stages, cudaStream_t st);
 // The attempt kernel (attempt.cu): whether it takes this batch, and its run.
-bool attempt_fits(const PropArgs& A, int method);
+bool attempt_fits(const PropArgs& A);
 cudaError_t launch_attempts(const PropArgs& A, const PipeBufs& P, ReplayRes& R, int method, cudaStream_t st,
                             double max_seconds);
 

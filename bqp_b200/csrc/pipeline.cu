@@ -367,11 +367,8 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
     GravLaunch G = gravity_launch(GT, A.n, device_sm_count(), gthreads, gslots);
     GravLaunch GF = check ? gravity_launch(A.sur.full, A.n, device_sm_count(), gthreads, gslots) : G;
     auto gker = pl_gravity_of(G), gker_full = pl_gravity_of(GF);
-    // the larger shared memory last: the two may be one kernel
-    cudaError_t e = cudaSuccess;
-    if (check && GF.smem < G.smem) e = gravity_ready(GF, gker_full);
-    if (e == cudaSuccess) e = gravity_ready(G, gker);
-    if (e == cudaSuccess && check && GF.smem >= G.smem) e = gravity_ready(GF, gker_full);
+    cudaError_t e = gravity_ready(G, gker);
+    if (e == cudaSuccess && check) e = gravity_ready(GF, gker_full);
     if (e != cudaSuccess) return e;
     e = upload_fixed_fit(A, user);
     if (e != cudaSuccess) return e;
@@ -476,7 +473,7 @@ cudaError_t launch_pipeline(const PropArgs& A, const PipeBufs& P, ReplayRes& R, 
                             int gravity_threads, int gravity_slots, KernelTimes* times) {
     if (A.n <= 0) return cudaSuccess;
     if (gravity_threads <= 0) gravity_threads = 256;
-    if (!times && gravity_threads == 256 && gravity_slots != 1 && gravity_slots != 2 && attempt_fits(A, method))
+    if (!times && gravity_threads == 256 && gravity_slots != 1 && gravity_slots != 2 && attempt_fits(A))
         return launch_attempts(A, P, R, method, st, max_seconds);
     switch (method) {
         case kDopri5: return run<kDopri5>(A, P, R, st, max_seconds, gravity_threads, gravity_slots, times);

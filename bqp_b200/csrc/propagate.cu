@@ -278,10 +278,8 @@ cudaError_t launch_rhs(const double* gtab, uint32_t tab_bytes, int use_smem, con
                        double* out, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     const size_t smem = use_smem ? tab_bytes : 0;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    cudaError_t e = cudaFuncSetAttribute(k_rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemLimit);
+    if (e != cudaSuccess) return e;
     const int threads = 256;
     int64_t blocks = (n + threads - 1) / threads;
     const int64_t cap = (int64_t)sm_count();
@@ -295,7 +293,7 @@ template <int M>
 static cudaError_t launch_prop_m(const PropArgs& A, int threads, int blocks, cudaStream_t st) {
     const size_t smem = A.use_smem ? A.tab_bytes : 0;
     cudaError_t e = cudaFuncSetAttribute(k_propagate<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(smem > 0 ? smem : 0));
+                                         (int)kSmemLimit);
     if (e != cudaSuccess) return e;
     k_propagate<M><<<blocks, threads, smem, st>>>(A);
     return cudaGetLastError();
