@@ -50,7 +50,7 @@ constexpr int kFourLanesRows = 25;
 
 // the table and the shares' sums, beside the static arrays (at_attempt's)
 constexpr size_t kAttemptStatic = 12 * 1024, kAttemptSmem = kSmemLimit - kAttemptStatic;
-static_assert(sizeof(uint64_t) + kAttemptRows / 32 * sizeof(EclWarpStore) + (4 * kAttemptRows + 7) * sizeof(int32_t) + 64 <=
+static_assert(sizeof(uint64_t) + kAttemptRows / 32 * sizeof(EclWarpStore) + (4 * kAttemptRows + 8) * sizeof(int32_t) + 64 <=
               kAttemptStatic);
 size_t attempt_smem_bytes(const GravTable& T, int shares) {
     return ((size_t)shares * 3 * kAttemptRows + kGravityTabPad) * sizeof(double) + T.bytes;
@@ -138,11 +138,15 @@ __device__ __forceinline__ void attempt_gravity_cells(const PipeBufs& P, const G
 // Launch number `at` of six: up to `rounds` attempts of the rows of list at % 2,
 // counted in count[at % 3]; rows that go on are appended to the other list and
 // count[(at + 1) % 3], and count[(at + 2) % 3] is cleared for the launch after
-// this one (nothing reads it any more).
+// this one (nothing reads it any more).  Once the call's wall-clock limit is
+// over no row makes another attempt: the rows go on to the next list as they
+// are, until the host ends them (over[at % 2] is the launch before's word, read
+// alike by every thread; over[(at + 1) % 2] is this one's).  `first`: one
+// attempt whatever the clock says.
 template <int M>
 __global__ void __launch_bounds__(kAttemptThreads, 1)
     at_attempt(const __grid_constant__ PropArgs A, const __grid_constant__ PipeBufs P, int at, int dense,
-               int rounds) {
+               int rounds, int first) {
     extern __shared__ __align__(16) double smem_dyn[];  // [shares][3][kAttemptRows] sums, the table
     __shared__ __align__(8) uint64_t bar;
     __shared__ EclWarpStore ecl_ws[kAttemptRows / 32];
@@ -150,8 +154,10 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
     __shared__ int32_t n_list[2][2], row_list[2][kAttemptRows];
     // the CTA's trajectories, of this attempt and the next; row r is slot b0 + r
     __shared__ int32_t trajs[2][kAttemptRows], n_traj[2];
+    __shared__ int32_t over;        // the call's wall-clock limit is over
     __shared__ int32_t four_lanes;  // exact density: the launch's rows a CTA are at most kFourLanesRows
     const int count = P.count[at % 3];
+    const bool none = !first && P.over[at & 1];  // no attempt in this launch
     const int per = (count + gridDim.x - 1) / gridDim.x;
     const int b0 = blockIdx.x * per;
     int rows = min(per, count - b0);
@@ -166,12 +172,16 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
     double* red = smem_dyn;
     double* tab = smem_dyn + shares * 3 * kAttemptRows;
     bool staged = true;
-    if (fp.gravity_on)
+    if (tid == 0) {
+        over = none;
+        if (none) P.over[(at & 1) ^ 1] = 1;
+    }
+    if (fp.gravity_on && !none)
         staged = stage_begin(&bar, A.grav.bytes, [&](auto copy) { copy(tab, A.grav.tab, A.grav.bytes); });
     const int stages = Tab<M>::S + (dense ? 1 : 0);
     __syncthreads();  // the trajectories are listed
     int round = 0;
-    for (; round < rounds && rows > 0; ++round) {
+    for (; round < rounds && rows > 0 && !over; ++round) {
         const int32_t* list = trajs[round & 1];
         if (tid == 0) n_traj[(round & 1) ^ 1] = 0;  // read again after the stages' barriers
         // the instants: part k of stage s of row r, the parts in different warps
@@ -238,6 +248,8 @@ __global__ void __launch_bounds__(kAttemptThreads, 1)
         if (warp * 32 < rows)
             control_warp<M>(A, P, tid < rows ? list[tid] : 0, b0 + tid, tid < rows, trajs[(round & 1) ^ 1],
                             &n_traj[(round & 1) ^ 1], ecl_ws[warp], dense);
+        // the clock, read by a warp that has no controller's rows
+        if (tid == kAttemptThreads - 1 && over_time(A, P)) over = P.over[(at & 1) ^ 1] = 1;
         __syncthreads();
         rows = n_traj[(round & 1) ^ 1];
     }
@@ -258,6 +270,9 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
     if (e != cudaSuccess) return e;
     const int blocks = (int)((A.n + kBlock - 1) / kBlock);
     const int ctas = (int)(A.n < device_sm_count() ? A.n : device_sm_count());
+    // launches that make an attempt whatever the clock says: as many as the
+    // stage kernels make before the host first looks at it
+    int unconditional = 4;
     return replay(
         P, R, user, max_seconds, false, false, [&](cudaStream_t st) { pl_init<M><<<blocks, kBlock, 0, st>>>(A, P); },
         [&](cudaStream_t st, cudaStream_t, const StreamOrder&) {
@@ -265,7 +280,8 @@ static cudaError_t run(const PropArgs& A, const PipeBufs& P, ReplayRes& R, cudaS
             for (int at = 0; at < 6; ++at) {
                 if (A.ordered) launch_times(A, P, M, at & 1, at % 3, Tab<M>::S + (dense ? 1 : 0), st);
                 at_attempt<M><<<ctas, kAttemptThreads, smem, st>>>(A, P, at, dense ? 1 : 0,
-                                                                  A.ordered ? 1 : kAttemptRounds);
+                                                                  A.ordered ? 1 : kAttemptRounds, unconditional > 0 ? 1 : 0);
+                if (unconditional > 0) --unconditional;
             }
         },
         [&](cudaStream_t st) { pl_abort<M><<<blocks, kBlock, 0, st>>>(A, P, 0); }, [] {});

@@ -70,6 +70,8 @@ struct PipeBufs {
     TrajState* st;        // [cap]
     int32_t* idx[2];      // active lists (slot -> trajectory), double-buffered
     int32_t* count;       // [2] active counts (attempt kernel: [3])
+    uint64_t* started;    // the device's clock at the call's first kernel, ns
+    int32_t* over;        // [2] attempt kernel: the wall-clock limit was over in the launch before
     double* k;            // [(S+1)][6][cap] stage derivatives
     double* sp;           // [6][cap] perturbed state of the stage (ECI)
     // what a stage needs of its instant alone, formed for several stages at

@@ -291,6 +291,8 @@ void pipeline_carve(PipeBufs& P, void* base, int64_t cap, int iau, int drag) {
     P.idx[0] = (int32_t*)take(c * 4);
     P.idx[1] = (int32_t*)take(c * 4);
     P.count = (int32_t*)take(3 * 4);
+    P.started = (uint64_t*)take(8);
+    P.over = (int32_t*)take(2 * 4);
     P.k = (double*)take((size_t)kStageBufs * 6 * c * 8);
     P.sp = (double*)take(6 * c * 8);
     P.iau = iau;

@@ -488,11 +488,20 @@ __device__ __forceinline__ void control_warp(const PropArgs& A, const PipeBufs& 
     append_active(next, next_count, traj, keep);  // whole warps take part in the ballot
 }
 
+// Whether the call's wall-clock limit is over, by the device's clock.
+__device__ __forceinline__ bool over_time(const PropArgs& A, const PipeBufs& P) {
+    return A.ctrl.max_kernel_ns > 0 && (int64_t)(global_ns() - *P.started) > A.ctrl.max_kernel_ns;
+}
+
 // --------------------------------------------------------------------- init
 template <int M>
 __global__ void __launch_bounds__(kBlock) pl_init(const __grid_constant__ PropArgs A, const __grid_constant__ PipeBufs P) {
     const int64_t traj = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool keep = false;
+    if (traj == 0) {
+        *P.started = global_ns();
+        P.over[0] = P.over[1] = 0;
+    }
     if (traj < A.n) {
         TrajState s;
         traj_begin(A, s, traj);

@@ -100,8 +100,8 @@ typedef struct bqp_force_config {
     double jb_drivers[9];   /* F10.7, F10.7bar, S10, S10bar, M10, M10bar, Y10, Y10bar, dTc (K) */
     int64_t max_steps;      /* per rectification segment (MAX_STEPS = 500000) */
     int64_t max_attempts;   /* device watchdog: step attempts per trajectory */
-    double max_kernel_seconds; /* watchdog: wall-clock limit of one propagation call (> 0);
-                                  rows not finished by then end with BQP_ST_WATCHDOG */
+    double max_kernel_seconds; /* watchdog: wall-clock limit of one propagation call (> 0); rows not
+                                  finished a few step attempts after it end with BQP_ST_WATCHDOG */
     int32_t engine;            /* BQP_ENGINE_* */
     int32_t gravity_threads;   /* threads per CTA of the gravity kernels, 32..256; 0 or 256: 256 at
                                   most, fewer where drag runs beside, and small batches in one
