@@ -17,11 +17,13 @@ by the device per trajectory.
   e2e    the same steps through the host-buffer C ABI call
          (bqp_propagate_final): H2D of the inputs and D2H of the results
          inside the timed region
-  roofline  the gravity kernel (pl_gravity), FP64: algorithmic flops =
-         force evals x F(70) (the reference gravity algorithm's flop count,
-         F(N) = 9(N+2)(N+3)/2 + 13N(N+1) + 9(N+1) + 60, FMA = 2) over the
-         kernel's summed CUDA-event time in the timed steps; peak = cuBLAS
-         DGEMM measured in this run
+  roofline  the gravity kernel (pl_gravity), FP64: force evals x the flops its
+         form of the field executes (FMA = 2; the reference's algorithm has
+         F(N) = 9(N+2)(N+3)/2 + 13N(N+1) + 9(N+1) + 60, about twice as many)
+         over the kernel's summed CUDA-event time in a second pass of the
+         steps; peak = cuBLAS DGEMM measured in this run.  `executed_slots`
+         counts instructions, a product or a sum as one FMA: the share of the
+         FP64 pipe's issue slots
   cpu_baseline  the C++ oracle (restatement of the reference CPU path) on a
          bounded sample, all host cores
 
@@ -78,7 +80,18 @@ def form_name(args) -> str:
 
 
 def f_of_n(n: int) -> float:
+    """Flops of the reference's gravity algorithm."""
     return 9 * (n + 2) * (n + 3) / 2 + 13 * n * (n + 1) + 9 * (n + 1) + 60
+
+
+def executed_field(n: int):
+    """(flops, FP64 instructions) of the plain FP64 field of order n as executed:
+    a column of L cells has 6 FMAs in its second row and 7 FMAs and 2 products
+    in each row below, and at its end 8 FMAs and 2 products."""
+    cols = n + 2
+    below = sum(max(length - 2, 0) for length in range(1, cols + 1))
+    fma, mul = 6 * (cols - 1) + 7 * below + 8 * cols, 2 * below + 2 * cols
+    return 2.0 * fma + mul, float(fma + mul)
 
 
 def parse(argv=None):
@@ -280,7 +293,7 @@ def run_reference(args):
 # DRAM bytes (read + write) per launch of the dominant kernel from one ncu
 # capture (profiles/pl_gravity_70x70.md: 37,888 rows, one launch), scaled by
 # the rows one launch of this run processes.
-TRAFFIC_CAPTURE = {"gravity": (1895424.0, 37888)}
+TRAFFIC_CAPTURE = {"gravity": (1888512.0, 37888)}
 
 
 def traffic_per_launch(kernel: str, rows: int):
@@ -603,9 +616,10 @@ def run_ours(args):
     line = None
     if rank == 0:
         peak = fp64_peak_tflops(torch, dev)
-        fN = f_of_n(ORDER)
+        # split precision: no such count; the reference's
+        fN, slots = executed_field(ORDER) if not args.split_degree else (f_of_n(ORDER), None)
         # dominant kernel: the gravity stage; every force evaluation is one
-        # gravity evaluation, F(70) algorithmic flops each
+        # gravity evaluation
         dom = "persistent" if args.engine == "persistent" else "gravity"
         dom_ms, dom_launches = ktimes[dom]
         achieved = prof_evals * fN / (dom_ms * 1e-3) / 1e12
@@ -636,7 +650,9 @@ def run_ours(args):
                          "frac": achieved / peak, "traffic": traffic_per_launch(dom, n),
                          "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (no FP64 figure in "
                                         "MEASURED_PEAKS.json)",
-                         "flops_per_eval": fN,
+                         "flops_per_eval": fN, "reference_flops_per_eval": f_of_n(ORDER),
+                         "executed_slots": None if slots is None else
+                         prof_evals * slots * 2.0 / (dom_ms * 1e-3) / 1e12 / peak,
                          "kernel": "pl_gravity<4>" if dom == "gravity" else f"k_propagate<{args.method.upper()}>",
                          "kernel_ms": dom_ms, "kernel_launches": dom_launches,
                          "kernel_timing": "second pass of the K steps with a CUDA event on each side of "
