@@ -16,6 +16,14 @@
 // default 26,527 -> 14,435; 200 rows over 5,400 s 37,658 -> 25,269; 1,024 rows
 // over a day on a 60 s grid 519,986 -> 249,360; 6,000 mixed rows 371,461 ->
 // 286,615; 1,500 rows with SRP 261,000 -> 173,479.
+//
+// Its limit of 64 rows a CTA is what its arrays hold.  There (9,472 rows, 600 s,
+// DOP853 at 1e-10, attempt kernel against stage kernels): 20x20 without drag
+// 4,458 us and 7,334, 70x70 without drag 12,974 and 15,960, 70x70 with the fitted
+// density 22,262 and 23,070, with the exact one 44,045 and 37,732; with SRP
+// 157,266 and 207,844 (3,000 s).  Only the exact density at 70x70 runs
+// slower here, from about 30 rows a CTA (32,411 and 30,860); it is 1.22 times
+// as fast at 16.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -39,7 +39,7 @@ struct PropArgs {
     int64_t* steps;                // [n] or null
     int64_t* evals;                // [n] or null
     unsigned long long* queue;     // work-queue head, zeroed before launch
-    const double* gtab;            // gravity table (global), FP64 cells (the Encke force call)
+    const double* gtab;            // gravity table (global), FP64 columns (the Encke force call)
     uint32_t tab_bytes;            // its size
     int32_t use_smem;
     GravTable grav;                // the gravity stage's table (plain or split precision)
@@ -47,14 +47,21 @@ struct PropArgs {
     ForceParams force;
     CtrlParams ctrl;
     const jb::JbFit* fit_host;     // host copy of *force.fit (null with it): the stage-synchronous
-                                   // drag kernel takes it by value, in kernel parameter space
+                                   // drag kernels read it from constant memory
     // Sigma-point rows.  At tight tolerances an adaptive step's length follows
     // the last bits of the force (in the GMST frame through its instant too, a
     // one-part Julian day of 40 us steps): rows then end up to 1e-8 km apart,
     // which the covariance, made of the rows' differences, shows at up to 2e-9
-    // of itself.  So for these rows the field and the density are added up in a
-    // fixed order of operations whatever kernel runs them: the cells'
-    // (GravTable::cells), and jb2008's with ln of each species (density()).
+    // of itself.  So in the stage-synchronous engine these rows keep one order of
+    // operations: the field's columns by the table of cells (GravTable::cells) in
+    // kGravityPartsMax runs, the density with ln of each species (density()).
+    // The attempt and the stage kernels give them the same bits.  The runs
+    // are fewer where a CTA's threads do not hold four groups of them
+    // (gravity_layout: two above 256 active rows a CTA, one above 512, at 256
+    // threads and 4 rows a lane; other gravity_threads and gravity_slots move
+    // these limits) or its shared memory their sums (order 79 and up), so there
+    // the order follows the batch's active rows, as any batch's does.  The
+    // persistent engine adds the columns one after the other (gravity_field).
     int32_t ordered;
     struct EclState* ecl;          // [n] eclipse coordinator state of SRP rows (null without SRP)
 };

@@ -156,7 +156,9 @@ int bqp_ctx_create(const char* coeff_text, int64_t text_len, const bqp_force_con
 int bqp_ctx_destroy(bqp_ctx* ctx);
 /* cudaStream_t to enqueue on (NULL: the legacy default stream). */
 int bqp_ctx_set_stream(bqp_ctx* ctx, void* cuda_stream);
-/* info[0]=order, [1]=table cells, [2]=table bytes, [3]=table staged in shared memory */
+/* info[0]=order, [1]=table cells, [2]=table bytes, [3]=the table fits in one CTA's shared
+ * memory (the persistent engine and the force call read a larger one from global memory, the
+ * gravity kernels share it among the CTAs of a cluster) */
 int bqp_ctx_info(const bqp_ctx* ctx, int64_t* info4);
 /* Worst relative error of the JB2008 sweep fits against the quadrature at
  * the check points (-1: no fit, the quadrature always runs). */
@@ -166,7 +168,11 @@ int bqp_ctx_info_fit(const bqp_ctx* ctx, double* worst_rel);
  * side of every kernel launch and add up the durations by kernel class
  * (BQP_KCLASS_*); the totals restart at zero.  While it is on, the
  * stage-synchronous engine waits for each graph replay before queueing the
- * next.  on == 0 stops recording and keeps the totals. */
+ * next, and runs its stage kernels one after the other: gravity with 256
+ * threads by default, also where drag otherwise runs beside it (128 threads),
+ * and also for a small batch that otherwise takes one kernel an attempt.  Its
+ * times are those of these kernels, not shares of an untimed call's.  on == 0
+ * stops recording and keeps the totals. */
 #define BQP_KCLASS_PREP 0       /* stage preparation (baseline, frame, third body) */
 #define BQP_KCLASS_GRAVITY 1    /* spherical-harmonic gravity */
 #define BQP_KCLASS_DRAG 2       /* JB2008 density and drag (both altitude lists) */
